@@ -95,6 +95,28 @@ def test_gemm_rows_do_not_depend_on_the_batch():
     assert torch.equal(k.gemm_simt(x[17:18].contiguous(), w, k.EPI_STORE_F32), full[17:18])
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16, 17, 64, 65, 129, 193, 260])
+@pytest.mark.parametrize("K_", [4, 36, 512, 516, 1544, 2051, 4096])
+def test_gemm_simt_rows_of_both_kernels_are_the_same_sums(M, K_):
+    """Up to 16 rows and more take different kernels; block edges, K that leaves spans or quarters short or empty, rows
+    that are no whole pieces of 16 bytes.  Error of a sum of K products in any order: at most K * 2^-24 of their
+    absolute sum, here far less (16 spans of two running sums)."""
+    k = K()
+    N = 145
+    x = torch.randn(M, K_, device=DEV)
+    w = torch.randn(N, K_, device=DEV)
+    ref = x.double() @ w.double().t()
+    bound = (x.double().abs() @ w.double().abs().t()) * (K_ / 32 + 32) * 2.0 ** -24
+    got = k.gemm_simt(x, w, k.EPI_STORE_F32)
+    assert ((got.double() - ref).abs() <= bound).all()
+    acc = torch.randn(M, N + 3, device=DEV)
+    before = acc.clone()
+    k.gemm_simt(x, w, k.EPI_ADD_F32, acc[:, :N])
+    assert torch.equal(acc[:, :N], before[:, :N] + got) and torch.equal(acc[:, N:], before[:, N:])
+    for at, n in ((M - 1, 1), (M // 2, M - M // 2), (0, min(M, 17))):
+        assert torch.equal(k.gemm_simt(x[at:at + n].contiguous(), w, k.EPI_STORE_F32), got[at:at + n])
+
+
 # --------------------------------------------------------------- rope + append
 def _paged(n_pages, hkv, hd, dtype, fill=float("nan")):
     return (torch.full((n_pages, hkv, 64, hd), fill, device=DEV, dtype=DT[dtype]),
