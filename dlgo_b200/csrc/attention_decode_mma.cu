@@ -20,8 +20,10 @@
 // The probabilities go from the score accumulators straight into the A registers of the second MMA
 // (rounded to bfloat16, as the prompt kernel does).
 //
-// A block takes one sequence, one kv head (8 of its query heads) and a slice of the pages; 2..8
-// slices form a thread-block cluster and combine through distributed shared memory.
+// Two kernels share that loop.  `attention_decode_mma_kernel`: a block takes one sequence, one kv head (8 of its query
+// heads) and a slice of the pages; 2..8 slices form a thread-block cluster and combine through distributed shared
+// memory.  `attention_decode_shares_kernel`: the blocks of a kv head share all keys of the step evenly, wherever the
+// sequences begin and end, so the longest sequence of a batch does not decide how long the launch takes.
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -345,6 +347,353 @@ __global__ void __launch_bounds__(DM_THREADS, HD <= 64 ? 4 : 2) attention_decode
   if (threadIdx.x == 0) TSTAMP(7);
 }
 
+// ------------------------------------------------------------------ even shares
+// Bound by the keys and values, which are read once.  The tiles (TK keys) of all sequences, one sequence after another,
+// are numbered through, and each of a kv head's blocks takes an equal run of them: as many blocks as are resident at
+// once, so that every SM streams until the end.  A run may hold several sequences or a part of one: at most its first
+// and its last sequence are shared with other blocks.  Their partial results go through scratch memory, and the block
+// that takes a sequence's last ticket adds them up; nobody waits for another block.  Every block works out the cut
+// from the positions (the step's own inputs) while its predecessor drains.
+// Measured on a B200: 32 sequences of 256 to 4,096 keys, 8 kv heads of 128 (301 MB) 61 us, 49 of them streaming at 6.1
+// TB/s; one slice per sequence 87 us, a cluster of two 85.  In a step at the 8B sizes 6.23 -> 5.16 ms, 3B sizes with 16
+// sequences of 64 to 2,048 keys 2.45 -> 2.11, 1B sizes with two of 14,000 to 17,800 1.06 -> 0.98 (37 slices combined by
+// a second kernel before).  Clusters stay where they leave a block two or three rounds: their sums meet faster (16
+// sequences of 128 to 1,024 keys, heads of 64: 9 us against 14).
+// Up to DS_SEGS sequences at a time go through one round: queries (rotated here where the projection's sum comes in,
+// new keys and values appended) to shared memory, the warps' tiles of all of them without a barrier, one merge.
+constexpr int DS_SEGS = 4;
+constexpr int DS_MIN_TILES = 8;       // a block's least run: two tiles a warp
+constexpr int DS_MAX_B = 2048;        // sequences (their first tiles lie in shared memory)
+
+__device__ int g_decode_append_error = 0;
+
+template <int HD> constexpr size_t shares_smem(int B, int gm) {
+  return (size_t)(B + 4) / 4 * 16 + (size_t)DS_SEGS * gm * HD * 2 + (size_t)DS_SEGS * DM_WARPS * gm * (HD + 4 + 2) * 4;
+}
+
+template <int HD, int NJ, bool SPLIT>
+__global__ void __launch_bounds__(DM_THREADS, HD <= 64 ? 4 : 2)
+attention_decode_shares_kernel(DecMmaParams p, int B, int* tickets) {
+  using T = __nv_bfloat16;
+  constexpr int TK = 8 * NJ, KK = HD / 16, NT = HD / 8, QV = HD / 32, RH = HD / 2;
+  constexpr int AR = HD + 4;            // floats from one output row to the next in shared memory
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int last[DS_SEGS], longest;
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r = lane >> 2, c = lane & 3;
+  const int G = p.Hq / p.Hkv;
+  const int kvh = blockIdx.y / p.n_gchunks, gc = blockIdx.y - kvh * p.n_gchunks;
+  const int GM = min(DM_GM, G), g0 = gc * DM_GM, GC = min(DM_GM, G - g0);
+  const int head0 = kvh * G + g0;
+  int* first = reinterpret_cast<int*>(smem);                                  // [B + 1] first tile of each sequence
+  T* q_s = reinterpret_cast<T*>(smem + (size_t)(B + 4) / 4 * 16);             // [DS_SEGS][GM][HD]
+  float* acc_s = reinterpret_cast<float*>(q_s + (size_t)DS_SEGS * GM * HD);   // [DS_SEGS][DM_WARPS][GM][AR]
+  float* ml_s = acc_s + (size_t)DS_SEGS * DM_WARPS * GM * AR;                 // [DS_SEGS][DM_WARPS][GM][2]
+
+  if (warp == 0) {
+    int sum = 0, most = 0;
+    if (lane == 0) first[0] = 0;
+    for (int b0 = 0; b0 < B; b0 += 32) {
+      int n = 0;
+      if (b0 + lane < B) {
+        const int pos = p.token_pos[b0 + lane];
+        n = pos / TK - first_visible(pos, p.window) / TK + 1;
+        most = max(most, n);
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, n, o);
+        if (lane >= o) n += up;
+      }
+      n += sum;
+      if (b0 + lane < B) first[b0 + lane + 1] = n;
+      sum = __shfl_sync(0xffffffffu, n, 31);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) longest = most;
+  }
+  __syncthreads();
+  const unsigned P = first[B];
+  // A block per sequence where the longest does not outlast the whole launch by more than sharing costs: a tile of one
+  // block takes some 0.5 us while all stream, the launch streams 6.5 MB/us, and parts, tickets and sums take 5 us.
+  // (Measured on a B200, a block per sequence / shares, us: 32 sequences of 2,048, heads of 128, 53 / 55; of 256 to
+  // 4,096 87 / 61; 16 of 64 to 2,048 42 / 20; 64 of 128 to 1,024, heads of 64, 21 / 23; of 128 to 4,096 68 / 55.)
+  const bool whole_only = B <= (int)gridDim.x &&
+      (float)longest * 0.5f <= (float)P * ((float)gridDim.y * TK * HD * 4 / 6.5e6f) + 5.f;
+  const unsigned nb = whole_only ? B : min(gridDim.x, max(1u, (P + DS_MIN_TILES - 1) / DS_MIN_TILES));   // (<= P: no run is empty)
+  if (blockIdx.x >= nb) return;
+  const bool narrow = P < 0xffffffffu / nb;           // (a division of 64 bits takes a microsecond's tenth)
+  auto start_of = [&](unsigned i) {
+    if (whole_only) return first[i];
+    return (int)(narrow ? i * P / nb : (unsigned)((unsigned long long)i * P / nb));
+  };
+  auto block_of = [&](unsigned tile) {
+    return (int)(narrow ? ((tile + 1) * nb - 1) / P : (unsigned)(((unsigned long long)(tile + 1) * nb - 1) / P));
+  };
+  const int lo = start_of(blockIdx.x), hi = start_of(blockIdx.x + 1);
+  int b = 0;
+  for (int step = 1024; step > 0; step >>= 1)                              // the sequence that holds tile lo
+    if (b + step < B && first[b + step] <= lo) b += step;
+  static_assert(DS_MAX_B <= 2 * 1024, "the search covers them");
+  // page numbers, and cosine and sine rows, into L1 before the wait
+  for (int s = b; s < B && first[s] < hi; ++s) {
+    const int pos = p.token_pos[s], rebase = first_visible(pos, p.window) / TK - first[s];
+    const int* row = p.page_table + (size_t)p.seq_slot[s] * p.max_pages;
+    const int pg0 = (max(lo, first[s]) + rebase) * TK / p.page_size, pg1 = (min(hi, first[s + 1]) - 1 + rebase) * TK / p.page_size;
+    for (int pg = pg0 + tid * 32; pg < pg1 + 32; pg += DM_THREADS * 32)
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(row + min(pg, pg1)));
+    constexpr int LN = (RH * 4 + 127) / 128;
+    if (p.parts != nullptr && tid >= 64 && tid < 64 + 2 * LN) {
+      const float* tbl = (tid - 64 < LN ? p.cos_t : p.sin_t) + (size_t)pos * RH;
+      asm volatile("prefetch.global.L1 [%0];" ::"l"((const char*)tbl + (size_t)((tid - 64) % LN) * 128));
+    }
+  }
+  pdl_wait();
+
+  for (; b < B && first[b] < hi; b += DS_SEGS) {
+    int ns = 1;
+    while (ns < DS_SEGS && b + ns < B && first[b + ns] < hi) ++ns;
+    // queries, and the new key and value where this block holds the sequence's last tile; four pairs a thread
+    constexpr int R4 = RH / 4;
+    for (int idx = tid; idx < ns * (GC + 1) * R4; idx += DM_THREADS) {
+      const int i = idx % R4 * 4, g = idx / R4 % (GC + 1), s = idx / (R4 * (GC + 1));
+      const bool fresh = g == GC;
+      if (fresh && (p.parts == nullptr || !p.write_cache || gc != 0 || first[b + s + 1] > hi)) continue;
+      T* dst = q_s + ((size_t)s * GM + g) * HD + i;
+      if (p.parts == nullptr) {
+        const T* src = p.q + (size_t)(b + s) * p.ldq + (size_t)(head0 + g) * HD + i;
+        *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(src);
+        *reinterpret_cast<uint2*>(dst + RH) = *reinterpret_cast<const uint2*>(src + RH);
+        continue;
+      }
+      const int pos = p.token_pos[b + s];
+      const float4 cs = *reinterpret_cast<const float4*>(p.cos_t + (size_t)pos * RH + i);
+      const float4 sn = *reinterpret_cast<const float4*>(p.sin_t + (size_t)pos * RH + i);
+      const float* src = p.parts + (size_t)(b + s) * p.ldq + (size_t)(fresh ? p.Hq + kvh : head0 + g) * HD + i;
+      auto sum4 = [&](const float* at) {
+        float4 x = __ldcg(reinterpret_cast<const float4*>(at));
+        for (int sl = 1; sl < p.S; ++sl) {          // slice order
+          const float4 u = __ldcg(reinterpret_cast<const float4*>(at + (size_t)sl * p.part_stride));
+          x.x += u.x; x.y += u.y; x.z += u.z; x.w += u.w;
+        }
+        return x;
+      };
+      float4 x0, x1, v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
+      int page = 0;
+      if (fresh) {
+        page = p.page_table[(size_t)p.seq_slot[b + s] * p.max_pages + pos / p.page_size];
+        if (page < 0) {               // a page that was never reserved: nothing is written
+          atomicExch(&g_decode_append_error, 1);
+          continue;
+        }
+      }
+      if (p.S == 1) {               // (all of a thread's loads in flight at once)
+        x0 = __ldcg(reinterpret_cast<const float4*>(src));
+        x1 = __ldcg(reinterpret_cast<const float4*>(src + RH));
+        if (fresh) {
+          v0 = __ldcg(reinterpret_cast<const float4*>(src + (size_t)p.Hkv * HD));
+          v1 = __ldcg(reinterpret_cast<const float4*>(src + (size_t)p.Hkv * HD + RH));
+        }
+      } else {
+        x0 = sum4(src);
+        x1 = sum4(src + RH);
+        if (fresh) {
+          v0 = sum4(src + (size_t)p.Hkv * HD);
+          v1 = sum4(src + (size_t)p.Hkv * HD + RH);
+        }
+      }
+      if (fresh) {
+        const size_t row = (((size_t)page * p.Hkv + kvh) * p.page_size + pos % p.page_size) * HD + i;
+        dst = const_cast<T*>(p.kpages) + row;
+        T* vd = const_cast<T*>(p.vpages) + row;
+        *reinterpret_cast<uint2*>(vd) = make_uint2(pack_bf16(v0.x, v0.y), pack_bf16(v0.z, v0.w));
+        *reinterpret_cast<uint2*>(vd + RH) = make_uint2(pack_bf16(v1.x, v1.y), pack_bf16(v1.z, v1.w));
+      }
+      *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(x0.x * cs.x - x1.x * sn.x, x0.y * cs.y - x1.y * sn.y),
+                                                  pack_bf16(x0.z * cs.z - x1.z * sn.z, x0.w * cs.w - x1.w * sn.w));
+      *reinterpret_cast<uint2*>(dst + RH) = make_uint2(pack_bf16(x0.x * sn.x + x1.x * cs.x, x0.y * sn.y + x1.y * cs.y),
+                                                       pack_bf16(x0.z * sn.z + x1.z * cs.z, x0.w * sn.w + x1.w * cs.w));
+      if (fresh) __threadfence_block();
+    }
+    __syncthreads();
+    for (int s = 0; s < ns; ++s) {
+      const int begin = max(lo, first[b + s]), end = min(hi, first[b + s + 1]);
+      const int pos = p.token_pos[b + s], t_begin = first_visible(pos, p.window);
+      const int rebase = t_begin / TK - first[b + s];        // to the sequence's own tile numbers
+      uint32_t qa[KK][2];
+#pragma unroll
+      for (int v = 0; v < QV; ++v) {
+        uint4 u = make_uint4(0u, 0u, 0u, 0u);
+        if (r < GC) u = *reinterpret_cast<const uint4*>(q_s + ((size_t)s * GM + r) * HD + c * (HD / 4) + v * 8);
+        qa[2 * v][0] = u.x; qa[2 * v][1] = u.y;
+        qa[2 * v + 1][0] = u.z; qa[2 * v + 1][1] = u.w;
+      }
+      float o[NT][2];
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) o[nt][0] = o[nt][1] = 0.f;
+      float m = -INFINITY, l = 0.f;
+      decode_attend_tiles<HD, NJ, SPLIT>(p.kpages, p.vpages, p.page_table + (size_t)p.seq_slot[b + s] * p.max_pages, p.Hkv,
+                                         kvh, p.page_size, 0, end + rebase, t_begin, pos + 1, p.scale,
+                                         begin + rebase + ((warp - (begin - lo)) & (DM_WARPS - 1)), DM_WARPS, lane, qa, o, m, l);
+      l += __shfl_xor_sync(0xffffffffu, l, 1);
+      l += __shfl_xor_sync(0xffffffffu, l, 2);
+      if (r < GC) {
+        float* as = acc_s + (((size_t)s * DM_WARPS + warp) * GM + r) * AR;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          as[(2 * c) * (HD / 8) + nt] = o[nt][0];            // (MMA column nt * 8 + 2c + e: see above)
+          as[(2 * c + 1) * (HD / 8) + nt] = o[nt][1];
+        }
+        if (c == 0) {
+          float* ml = ml_s + ((s * DM_WARPS + warp) * GM + r) * 2;
+          ml[0] = m;
+          ml[1] = l;
+        }
+      }
+    }
+    __syncthreads();
+    bool shared_any = false;
+    for (int s = 0; s < ns; ++s) shared_any |= first[b + s] < lo || first[b + s + 1] > hi;
+    constexpr int H4 = HD / 4;
+    auto store4 = [&](int seq, int g, int d, float4 a, float ll, float mm) {
+      float v[4] = {a.x, a.y, a.z, a.w}, l4 = ll;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        l4 = ll;
+        join_sink(v[e], l4, mm, p.sink, head0 + g);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] /= l4;
+      *reinterpret_cast<uint2*>(p.out + (size_t)seq * p.ldo + (size_t)(head0 + g) * HD + d) =
+          make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+    };
+    for (int idx = tid; idx < ns * GC * H4; idx += DM_THREADS) {
+      const int d = idx % H4 * 4, g = idx / H4 % GC, s = idx / (H4 * GC);
+      const float* ml = ml_s + (s * DM_WARPS * GM + g) * 2;
+      const float* as = acc_s + ((size_t)s * DM_WARPS * GM + g) * AR + d;
+      float mm = -INFINITY, ll = 0.f;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < DM_WARPS; ++w) mm = fmaxf(mm, ml[w * GM * 2]);
+#pragma unroll
+      for (int w = 0; w < DM_WARPS; ++w) {
+        const float mw = ml[w * GM * 2];
+        const float cw = mw == -INFINITY ? 0.f : expf(mw - mm);
+        const float4 u = *reinterpret_cast<const float4*>(as + w * GM * AR);
+        a.x = fmaf(cw, u.x, a.x); a.y = fmaf(cw, u.y, a.y); a.z = fmaf(cw, u.z, a.z); a.w = fmaf(cw, u.w, a.w);
+        ll = fmaf(cw, ml[w * GM * 2 + 1], ll);
+      }
+      if (first[b + s] >= lo && first[b + s + 1] <= hi) {
+        store4(b + s, g, d, a, ll, mm);
+      } else {        // a block shares at most two sequences: one that began before its run, one that begins in it
+        const size_t at = (((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 2 + (first[b + s] >= lo ? 1 : 0)) * GM + g;
+        *reinterpret_cast<float4*>(p.part_acc + at * HD + d) = a;
+        if (d == 0) *reinterpret_cast<float2*>(p.part_ml + at * 2) = make_float2(mm, ll);
+      }
+    }
+    if (shared_any) {
+      __syncthreads();
+      if (tid < ns) {
+        const int seq = b + tid;
+        int mine = 0;
+        if (first[seq] < lo || first[seq + 1] > hi) {
+          const int n = block_of(first[seq + 1] - 1) - block_of(first[seq]) + 1;
+          int* ticket = tickets + (size_t)seq * gridDim.y + blockIdx.y;
+          __threadfence();            // the block's parts, behind the barrier, before the ticket
+          if (atomicAdd(ticket, 1) == n - 1) {
+            *ticket = 0;              // for the next launch
+            mine = 1;
+          }
+          __threadfence();
+        }
+        last[tid] = mine;
+      }
+      __syncthreads();
+    }
+    for (int s = 0; s < ns; ++s) {
+      const int seq = b + s;
+      const bool whole = first[seq] >= lo && first[seq + 1] <= hi;
+      if (!whole && !last[s]) continue;           // (block-uniform)
+      if (!whole) {
+        const int i0 = block_of(first[seq]), n = block_of(first[seq + 1] - 1) - i0 + 1;
+        // a thread per four dimensions, or 2, 4, 8 threads that share the parts; four parts in flight each
+        const int cols = GC * H4;
+        int tpc = 1;
+        while (tpc < 8 && cols * tpc * 2 <= DM_THREADS) tpc *= 2;
+        for (int c0 = 0; c0 < cols; c0 += DM_THREADS / tpc) {
+          const int col = c0 + tid / tpc;
+          const int g = min(col, cols - 1) / H4, d = min(col, cols - 1) % H4 * 4;
+          float mm = -INFINITY, ll = 0.f;
+          float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int k0 = tid % tpc; k0 < n; k0 += 4 * tpc) {
+            float2 ml[4];
+            float4 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int k = k0 + j * tpc;
+              const size_t at = (((size_t)blockIdx.y * gridDim.x + i0 + min(k, n - 1)) * 2 + (k == 0 ? 1 : 0)) * GM + g;
+              ml[j] = k < n ? __ldcg(reinterpret_cast<const float2*>(p.part_ml) + at) : make_float2(-INFINITY, 0.f);
+              v[j] = k < n ? __ldcg(reinterpret_cast<const float4*>(p.part_acc + at * HD + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            float top = mm;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) top = fmaxf(top, ml[j].x);
+            if (top == -INFINITY) continue;
+            const float keep = mm == -INFINITY ? 0.f : expf(mm - top);
+            mm = top;
+            ll *= keep; a.x *= keep; a.y *= keep; a.z *= keep; a.w *= keep;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float w = ml[j].x == -INFINITY ? 0.f : expf(ml[j].x - top);
+              ll = fmaf(w, ml[j].y, ll);
+              a.x = fmaf(w, v[j].x, a.x); a.y = fmaf(w, v[j].y, a.y);
+              a.z = fmaf(w, v[j].z, a.z); a.w = fmaf(w, v[j].w, a.w);
+            }
+          }
+          for (int o = tpc >> 1; o > 0; o >>= 1) {
+            const float m2 = __shfl_xor_sync(0xffffffffu, mm, o), top = fmaxf(mm, m2);
+            const float k1 = mm == -INFINITY ? 0.f : expf(mm - top), k2 = m2 == -INFINITY ? 0.f : expf(m2 - top);
+            mm = top;
+            ll = ll * k1 + __shfl_xor_sync(0xffffffffu, ll, o) * k2;
+            a.x = a.x * k1 + __shfl_xor_sync(0xffffffffu, a.x, o) * k2;
+            a.y = a.y * k1 + __shfl_xor_sync(0xffffffffu, a.y, o) * k2;
+            a.z = a.z * k1 + __shfl_xor_sync(0xffffffffu, a.z, o) * k2;
+            a.w = a.w * k1 + __shfl_xor_sync(0xffffffffu, a.w, o) * k2;
+          }
+          if (col < cols && tid % tpc == 0) store4(seq, g, d, a, ll, mm);
+        }
+      }
+      if (p.clear_parts) {      // every block of this sequence has read its sums: zero again for the next step
+        float4* row = reinterpret_cast<float4*>(const_cast<float*>(p.parts) + (size_t)seq * p.ldq);
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = tid; i < GC * H4; i += DM_THREADS) row[(size_t)head0 * H4 + i] = zero;
+        if (gc == 0)
+          for (int i = tid; i < 2 * H4; i += DM_THREADS) row[(size_t)(p.Hq + kvh + (i < H4 ? 0 : p.Hkv)) * H4 + i % H4] = zero;
+      }
+    }
+    __syncthreads();            // the round's shared memory is free again
+  }
+}
+
+// blocks of a kv head (or chunk of its heads) in a launch of even shares: as many as are resident at once
+inline int shares_blocks(int hd, int heads) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int n = (hd <= 64 ? 4 : 2) * sms / heads;
+  return n < 1 ? 1 : n;
+}
+
+template <int HD, bool SPLIT>
+int launch_decode_shares(const DecMmaParams& p, int B, int* tickets, cudaStream_t stream) {
+  const int heads = p.Hkv * p.n_gchunks, G = p.Hq / p.Hkv;
+  const size_t smem = shares_smem<HD>(B, G < DM_GM ? G : DM_GM);
+  cudaFuncSetAttribute((const void*)attention_decode_shares_kernel<HD, 4, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  launch_kernel(attention_decode_shares_kernel<HD, 4, SPLIT>, dim3(shares_blocks(HD, heads), heads), dim3(DM_THREADS), smem, stream, p, B,
+                tickets);
+  return launch_status();
+}
+
 template <int HD, int NJ, bool SPLIT>
 int launch_decode_mma(const DecMmaParams& p, int B, cudaStream_t stream) {
   dim3 grid(B, p.Hkv * p.n_gchunks, p.n_splits);
@@ -372,11 +721,29 @@ DLGO_EXPORT int dlgo_attention_decode_mma_takes(int hd, int page_size, int n_spl
   return (hd == 64 || hd == 128) && page_size % 32 == 0 && n_splits >= 1 && n_splits <= 65535;
 }
 
+// 1 if an append of a launch of even shares was skipped since the last call because its position had no page (clears the
+// word).
+DLGO_EXPORT int dlgo_attention_decode_mma_error() {
+  int v = 0, zero = 0;
+  if (cudaMemcpyFromSymbol(&v, g_decode_append_error, sizeof(int)) != cudaSuccess) return -1;
+  if (v) cudaMemcpyToSymbol(g_decode_append_error, &zero, sizeof(int));
+  return v;
+}
+
+// Floats of scratch that a launch of even shares needs.
+DLGO_EXPORT long long dlgo_attention_decode_shares_scratch(int Hq, int Hkv, int hd) {
+  if (Hq <= 0 || Hkv <= 0 || Hq % Hkv) return 0;
+  const int G = Hq / Hkv, heads = Hkv * ((G + DM_GM - 1) / DM_GM), gm = G < DM_GM ? G : DM_GM;
+  return (long long)heads * shares_blocks(hd, heads) * 2 * gm * (hd + 2);
+}
+
 // q[B, .] bf16 (row stride ldq, head h at column h * hd), one token per sequence at position
 // token_pos[b] whose key and value are already in the cache; out[B, .] bf16 (row stride ldo).
 // Or, with `parts` ([S][B][ldq] fp32, slice stride part_stride floats: the unsummed K-slices of the q | k | v
 // projection) and cos/sin tables [positions][hd / 2]: q is null, the kernel sums, rotates (whole head,
 // pairs (i, i + hd/2)) and, with write_cache, appends the token's key and value itself.
+// n_splits 0: even shares of all sequences' keys (at most 2,048 sequences, 32 keys per tile); `scratch` as above,
+// `tickets` [B * Hkv * ceil(Hq / Hkv / 8)] zero, and left zero.
 // keys_per_tile: 16 or 32 keys per warp iteration.  `sink` [Hq] fp32 or null: joins the denominator.  `split`:
 // probabilities meet the values as two bfloat16 terms (16 bits of mantissa).
 DLGO_EXPORT int dlgo_attention_decode_mma(const void* q, int B, int ldq, const void* kpages, const void* vpages,
@@ -385,10 +752,15 @@ DLGO_EXPORT int dlgo_attention_decode_mma(const void* q, int B, int ldq, const v
                                           int page_size, int n_splits, int window, float scale, int keys_per_tile,
                                           float* scratch, const float* parts, int S, long long part_stride,
                                           const float* cos_t, const float* sin_t, int write_cache, int clear_parts,
-                                          const float* sink, int split, cudaStream_t stream) {
+                                          const float* sink, int split, int* tickets, cudaStream_t stream) {
   if (B <= 0) return DLGO_OK;
   if (Hq <= 0 || Hkv <= 0 || Hq % Hkv) return DLGO_ERR_SIZE;
-  if (!dlgo_attention_decode_mma_takes(hd, page_size, n_splits)) return DLGO_ERR_SIZE;
+  const bool shares = n_splits == 0;
+  if (!dlgo_attention_decode_mma_takes(hd, page_size, shares ? 1 : n_splits)) return DLGO_ERR_SIZE;
+  if (shares && (B > DS_MAX_B || keys_per_tile != 32 || scratch == nullptr || tickets == nullptr)) return DLGO_ERR_SIZE;
+  if (shares && (((uintptr_t)scratch & 15) || ((uintptr_t)out & 7) || (ldo & 3) ||
+                 (parts != nullptr && (((uintptr_t)cos_t | (uintptr_t)sin_t) & 15))))
+    return DLGO_ERR_ALIGN;
   if (keys_per_tile != 16 && keys_per_tile != 32) return DLGO_ERR_SIZE;
   if (n_splits > 8 && scratch == nullptr) return DLGO_ERR_SIZE;
   if ((ldq & 7) || ((uintptr_t)kpages & 15) || ((uintptr_t)vpages & 15)) return DLGO_ERR_ALIGN;
@@ -415,6 +787,14 @@ DLGO_EXPORT int dlgo_attention_decode_mma(const void* q, int B, int ldq, const v
   p.write_cache = write_cache;
   p.clear_parts = clear_parts;
   p.sink = sink;
+  if (shares) {
+    const int heads = Hkv * p.n_gchunks, gm = G < DM_GM ? G : DM_GM;
+    if (heads > 65535) return DLGO_ERR_SIZE;
+    p.part_acc = scratch;
+    p.part_ml = scratch + (size_t)heads * shares_blocks(hd, heads) * 2 * gm * hd;
+    if (hd == 64) return split ? launch_decode_shares<64, true>(p, B, tickets, stream) : launch_decode_shares<64, false>(p, B, tickets, stream);
+    return split ? launch_decode_shares<128, true>(p, B, tickets, stream) : launch_decode_shares<128, false>(p, B, tickets, stream);
+  }
   p.part_acc = n_splits > 8 ? scratch : nullptr;
   p.part_ml = n_splits > 8 ? scratch + (size_t)B * Hq * n_splits * hd : nullptr;
   if ((long long)Hkv * p.n_gchunks > 65535) return DLGO_ERR_SIZE;

@@ -2097,7 +2097,8 @@ def check_device_errors() -> None:
         if v != 0:
             raise KernelError("a token's position had no page in the cache's table (persistent decode kernel)")
     for lib, fn in (("rope_append", "dlgo_rope_append_error"), ("headnorm_rope", "dlgo_headnorm_rope_error"),
-                    ("wholenorm_append", "dlgo_wholenorm_append_error")):
+                    ("wholenorm_append", "dlgo_wholenorm_append_error"),
+                    ("attention_decode_mma", "dlgo_attention_decode_mma_error")):
         if lib in build._loaded and getattr(build._loaded[lib], fn)() != 0:
             raise KernelError("a token's position had no page in the cache's table: its keys and values were not "
                               "stored and the step's results are invalid")
@@ -2117,6 +2118,16 @@ def attention_decode_mma_fuses_rope(num_heads: int, num_kv_heads: int, head_dim:
     return rotary_dim == head_dim and not interleaved and num_heads // num_kv_heads <= 8
 
 
+SHARES_MAX_SEQUENCES = 2048      # of attention_decode_mma with n_splits 0
+
+
+def attention_decode_shares_scratch(num_heads: int, num_kv_heads: int, head_dim: int) -> int:
+    """Floats of scratch of :func:`attention_decode_mma` with ``n_splits`` 0."""
+    fn = _lib("attention_decode_mma").dlgo_attention_decode_shares_scratch
+    fn.restype = ctypes.c_longlong
+    return int(fn(_i(num_heads), _i(num_kv_heads), _i(head_dim)))
+
+
 def attention_decode_mma(q: Optional[torch.Tensor], ldq: int, B: int, kpages: torch.Tensor, vpages: torch.Tensor,
                          page_table: torch.Tensor, seq_slot: torch.Tensor, token_pos: torch.Tensor,
                          out: torch.Tensor, num_heads: int, num_kv_heads: int, head_dim: int, scale: float,
@@ -2124,9 +2135,11 @@ def attention_decode_mma(q: Optional[torch.Tensor], ldq: int, B: int, kpages: to
                          scratch: Optional[torch.Tensor] = None, parts: Optional[torch.Tensor] = None,
                          cos: Optional[torch.Tensor] = None, sin: Optional[torch.Tensor] = None,
                          write_cache: bool = True, clear_parts: bool = False, sink: Optional[torch.Tensor] = None,
-                         split: bool = False) -> torch.Tensor:
+                         split: bool = False, tickets: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Attention of one new token per sequence over its cached keys and values, bfloat16, on the
-    tensor cores (mma.sync); 2..8 slices combine inside a thread-block cluster, more go through
+    tensor cores (mma.sync).  ``n_splits`` 0: the blocks of a head share the keys of all sequences evenly
+    (``scratch``: ``attention_decode_shares_scratch`` floats; ``tickets``: a zero int32 per sequence and chunk of 8
+    heads of a kv head, left zero).  Else as many page slices per sequence: 2..8 slices combine inside a thread-block cluster, more go through
     ``scratch`` (``attention_scratch_floats`` floats) and a second kernel.  With ``parts`` (the q|k|v
     projection as fp32 [slices, sequences, columns], unrotated) the kernel sums the slices, rotates q and k
     and appends k and v itself; ``clear_parts`` (one slice, at most 8 page slices): the sum is left zero.  ``sink``
@@ -2162,16 +2175,22 @@ def attention_decode_mma(q: Optional[torch.Tensor], ldq: int, B: int, kpages: to
     if parts is None and clear_parts:
         raise KernelError("attention_decode_mma: clear_parts goes with parts")
     page_size = kpages.shape[-2]
-    if n_splits > 8:
-        need = attention_scratch_floats(B, num_heads, head_dim, n_splits)
+    if n_splits == 0 or n_splits > 8:
+        need = (attention_scratch_floats(B, num_heads, head_dim, n_splits) if n_splits else
+                attention_decode_shares_scratch(num_heads, num_kv_heads, head_dim))
         if scratch is None or scratch.dtype != torch.float32 or scratch.numel() < need:
             raise KernelError(f"attention_decode_mma: {n_splits} slices need {need} floats of scratch")
+    if n_splits == 0:
+        _need(tickets, torch.int32, "tickets")
+        if tickets.numel() < B * num_kv_heads * ((num_heads // num_kv_heads + 7) // 8):
+            raise KernelError("attention_decode_mma: a ticket per sequence and chunk of heads")
     st = _lib("attention_decode_mma").dlgo_attention_decode_mma(
         _ptr(q), _i(B), _i(ldq), _ptr(kpages), _ptr(vpages), _ptr(page_table), _i(page_table.shape[1]),
         _ptr(seq_slot), _ptr(token_pos), _ptr(out), _i(out.stride(0)), _i(num_heads), _i(num_kv_heads), _i(head_dim),
         _i(page_size), _i(n_splits), _i(window), _f(scale), _i(keys_per_tile),
-        _ptr(scratch if n_splits > 8 else None), _ptr(parts), _i(S), _ll(part_stride), _ptr(cos), _ptr(sin),
-        _i(1 if write_cache else 0), _i(1 if clear_parts else 0), _ptr(sink), _i(1 if split else 0), _stream())
+        _ptr(scratch if n_splits == 0 or n_splits > 8 else None), _ptr(parts), _i(S), _ll(part_stride), _ptr(cos), _ptr(sin),
+        _i(1 if write_cache else 0), _i(1 if clear_parts else 0), _ptr(sink), _i(1 if split else 0),
+        _ptr(tickets if n_splits == 0 else None), _stream())
     _check(st, "attention_decode_mma", 2 if n_splits > 8 else 1)
     return out
 

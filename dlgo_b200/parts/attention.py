@@ -25,6 +25,7 @@ from .linear import ADD_F32, STORE, STORE_F32, Linear, stack_rows
 from .registry import MIXERS
 
 _CLUSTER_MAX = int(os.environ.get("DLGO_ATTN_CLUSTER_MAX", 8))     # slices up to this many combine in a cluster
+_SHARES = int(os.environ.get("DLGO_ATTN_SHARES", 1))         # even shares of the step's keys where they are better (0: slices)
 _MMA_KEYS = int(os.environ.get("DLGO_ATTN_MMA_KEYS", 32))    # keys per warp iteration of the tensor-core decode kernel (0: off)
 # few tokens: the projection's K-slices meet in one fp32 sum (reductions at the memory) that is zero between steps
 _QKV_SUM = int(os.environ.get("DLGO_ATTN_QKV_SUM", 1))
@@ -138,8 +139,8 @@ class GQAAttention(Mixer):
                                          cache.page_size))
 
     def _decode_plan(self, ctx: Any, cache: Any, act: torch.dtype):
-        """(decode kernel?, tensor-core decode kernel?, page slices, scratch, counters, pages of the longest
-        sequence) for this step's attention."""
+        """(decode kernel?, tensor-core decode kernel?, page slices (0: even shares), scratch, counters, pages of the
+        longest sequence) for this step's attention."""
         T = ctx.n_tokens
         group = self.num_heads // self.num_kv_heads
         longest = ctx.capacity if ctx.captured else ctx.max_len
@@ -148,6 +149,17 @@ class GQAAttention(Mixer):
         n_splits, scratch, counters = self._decode_slices(ctx, cache, T, group, pages) if decode_kernel else (1, None, None)
         mma = (decode_kernel and _MMA_KEYS > 0 and
                K.attention_decode_mma_takes(act, self.head_dim, cache.page_size, n_splits))
+        # Even shares of all sequences' keys (n_splits 0) where a sequence would get few slices, so that the longest
+        # decides how long the launch takes, or more than a cluster holds.  Measured on a B200 in a whole step, ms, slices
+        # / shares: 8B sizes, 32 sequences (1 slice) 6.23 / 5.16; 3B, 16 (2) 2.45 / 2.11; 1B, two long ones (37) 1.06 /
+        # 0.98.  Four slices are better at heads of 128 (8B, 8 sequences of up to 1,024 keys: 12 us a layer / 15), and
+        # at heads of 64, whose blocks are twice as many, one (1B, 64 of up to 1,024 keys: 1.200 ms / 1.211) and two (32: 13
+        # us / 16).
+        if (mma and _SHARES and _MMA_KEYS == 32 and T <= K.SHARES_MAX_SEQUENCES and
+                (n_splits > 8 or (n_splits <= 3 and self.head_dim > 64))):
+            n_splits = 0
+            scratch = ctx.scratch("attention", K.attention_decode_shares_scratch(self.num_heads, self.num_kv_heads, self.head_dim))
+            counters = ctx.zeros("attention_tickets", T * self.num_kv_heads * ((group + 7) // 8))
         return decode_kernel, mma, n_splits, scratch, counters, pages
 
     def _attend(self, qkv: torch.Tensor, ctx: Any, cache: Any, out: torch.Tensor, decode_kernel: bool, mma: bool,
@@ -160,7 +172,8 @@ class GQAAttention(Mixer):
         if mma:
             K.attention_decode_mma(qkv, qkv.stride(0), T, cache.keys, cache.values, cache.page_table, ctx.seq_slot,
                                    ctx.token_pos, out, self.num_heads, self.num_kv_heads, self.head_dim, self.scale,
-                                   self.span(), n_splits, _MMA_KEYS, scratch, sink=self.sink, split=self.split_weights)
+                                   self.span(), n_splits, _MMA_KEYS, scratch, sink=self.sink, split=self.split_weights,
+                                   tickets=counters)
         elif decode_kernel:
             K.attention_decode(qkv, qkv.stride(0), T, cache.keys, cache.values, cache.page_table, ctx.seq_slot,
                                ctx.token_pos, out, self.num_heads, self.num_kv_heads, self.head_dim, self.scale,
@@ -214,17 +227,17 @@ class GQAAttention(Mixer):
             # few tokens: the projection's K-slices add themselves, at the memory, into one fp32 sum that is zero
             # between steps; whoever rotates reads it once and leaves zeros behind
             qkv_sum = ctx.zeros(f"qkv_sum{n_cols}", T * n_cols, torch.float32)[:T * n_cols].view(1, T, n_cols)
-            # (heads of 64 only: at 128 the kernel is at its register limit and the fused form measured 2 to 3 %
+            # (slices: heads of 64 only; at 128 that kernel is at its register limit and the fused form measured 2 to 3 %
             # slower in a whole step at the layer sizes of Llama 3.2 3B and 3.1 8B, batch 8)
-            fuse = (mma and _FUSE_ROPE and n_splits <= 8 and self.head_dim <= _FUSE_ROPE_MAX_HEAD and
+            fuse = (mma and _FUSE_ROPE and n_splits <= 8 and (n_splits == 0 or self.head_dim <= _FUSE_ROPE_MAX_HEAD) and
                     K.attention_decode_mma_fuses_rope(self.num_heads, self.num_kv_heads, self.head_dim, rot, inter))
             self.wqkv(x, ADD_F32, qkv_sum[0])
             if fuse:
                 # the decode kernel rotates, appends and clears itself: no launch for the rotation
                 K.attention_decode_mma(None, n_cols, T, cache.keys, cache.values, cache.page_table, ctx.seq_slot,
                                        ctx.token_pos, out, self.num_heads, self.num_kv_heads, self.head_dim,
-                                       self.scale, self.span(), n_splits, _MMA_KEYS, None, qkv_sum, cos, sin,
-                                       cache.writes, clear_parts=True)
+                                       self.scale, self.span(), n_splits, _MMA_KEYS, scratch, qkv_sum, cos, sin,
+                                       cache.writes, clear_parts=True, tickets=counters)
                 rotated = True
             else:
                 qkv = torch.empty((T, n_cols), dtype=x.dtype, device=x.device)

@@ -241,6 +241,15 @@ def _attention_case(dtype, hq, hkv, hd, seqs, window=0, n_splits=1, decode=False
             k.attention_decode_mma(qbuf, ld, T_, kp, vp, pt.to(DEV), torch.tensor(slots, dtype=torch.int32, device=DEV),
                                    torch.tensor(pos, dtype=torch.int32, device=DEV), out, hq, hkv, hd,
                                    1.0 / math.sqrt(hd), window, n_splits, keys, scratch if n_splits > 8 else None)
+    elif kernel == "shares":
+        tickets = torch.zeros(T_ * hkv * ((hq // hkv + 7) // 8), dtype=torch.int32, device=DEV)
+        scratch = torch.full((k.attention_decode_shares_scratch(hq, hkv, hd),), float("nan"), device=DEV)
+        for _ in range(2):      # twice: the tickets must be left ready for the next call
+            out.fill_(float("nan"))
+            k.attention_decode_mma(qbuf, ld, T_, kp, vp, pt.to(DEV), torch.tensor(slots, dtype=torch.int32, device=DEV),
+                                   torch.tensor(pos, dtype=torch.int32, device=DEV), out, hq, hkv, hd,
+                                   1.0 / math.sqrt(hd), window, 0, 32, scratch, tickets=tickets)
+        assert int(tickets.abs().sum()) == 0
     elif kernel == "decode":
         assert all(n == 1 for _, n in seqs) and k.attention_decode_takes(DT[dtype], hd, 64)
         # three ways to combine slices: a cluster (no scratch, up to 8 slices), the last slice (scratch and
@@ -1059,3 +1068,59 @@ def test_tensor_core_decode_attention_reads_and_clears_the_projections_sum(hq, h
     torch.testing.assert_close(got[True][0], got[False][0], atol=2e-2, rtol=2e-2)
     torch.testing.assert_close(got[True][1], got[False][1], atol=1e-2, rtol=8e-3)
     torch.testing.assert_close(got[True][2], got[False][2], atol=1e-2, rtol=8e-3)
+
+
+@pytest.mark.parametrize("hq,hkv,hd", [(8, 2, 64), (3, 1, 128), (20, 1, 64), (2, 2, 128)])
+@pytest.mark.parametrize("lens", [[1], [32], [33, 1, 64, 65], [3000, 5], [1] * 70, [900, 40, 41, 39, 700, 2, 1, 1, 64, 31]])
+@pytest.mark.parametrize("window", [0, 70])
+def test_decode_attention_in_even_shares(hq, hkv, hd, lens, window):
+    """Runs that hold a part of a sequence, one, or more than a round's; fewer tiles than blocks; a window that begins
+    inside a tile, whose earlier pages are gone.  (Outputs are rounded to bfloat16, as are the probabilities.)"""
+    out, ref = _attention_case("bfloat16", hq, hkv, hd, [(n - 1, 1) for n in lens], n_splits=0, decode=True, kernel="shares",
+                               window=window, dead_pages=bool(window))
+    torch.testing.assert_close(out, ref, atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("hq,hkv,hd,S", [(32, 8, 64, 1), (24, 8, 128, 1), (8, 1, 64, 3)])
+@pytest.mark.parametrize("lens", [[300, 1, 64, 65, 640, 129], [640], [7] * 40])
+def test_decode_attention_in_even_shares_rotates_appends_and_clears(hq, hkv, hd, S, lens):
+    # against rope_append (on the sum) followed by the kernel fed with the finished q
+    from dlgo_b200.parts.rope import RotaryEmbedding
+    k = K()
+    torch.manual_seed(hd + S)
+    cos, sin = (t.to(DEV) for t in RotaryEmbedding(hd, hd, 10000.0, 700, "split_half").tables())
+    B = len(lens)
+    pages_per = [(n + 63) // 64 for n in lens]
+    n_pages = sum(pages_per) + 1
+    perm = torch.randperm(n_pages).tolist()
+    pt = torch.full((B, max(pages_per)), -1, dtype=torch.int32)
+    for i, n in enumerate(pages_per):
+        for pg in range(n):
+            pt[i, pg] = perm.pop()
+    pt = pt.to(DEV)
+    ld = (hq + 2 * hkv) * hd
+    parts = torch.randn(S, B, ld, device=DEV) * 0.6
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV)
+    seq = torch.arange(B, dtype=torch.int32, device=DEV)
+    tickets = torch.zeros(B * hkv, dtype=torch.int32, device=DEV)
+    scratch = torch.full((k.attention_decode_shares_scratch(hq, hkv, hd),), float("nan"), device=DEV)
+    got = {}
+    for fused in (False, True):
+        torch.manual_seed(1)
+        kp = torch.randn(n_pages, hkv, 64, hd, device=DEV).to(torch.bfloat16)
+        vp = torch.randn(n_pages, hkv, 64, hd, device=DEV).to(torch.bfloat16)
+        out = torch.full((B, hq * hd), float("nan"), device=DEV, dtype=torch.bfloat16)
+        work = parts.clone()
+        if not fused:
+            qkv = torch.empty(B, ld, device=DEV, dtype=torch.bfloat16)
+            k.rope_append(qkv, cos, sin, pos, seq, seq, pt, kp, vp, hq, hkv, hd, hd, False, True, work)
+            k.attention_decode_mma(qkv, ld, B, kp, vp, pt, seq, pos, out, hq, hkv, hd, hd ** -0.5, 0, 1, 32)
+        else:
+            k.attention_decode_mma(None, ld, B, kp, vp, pt, seq, pos, out, hq, hkv, hd, hd ** -0.5, 0, 0, 32,
+                                   scratch, work, cos, sin, True, clear_parts=S == 1, tickets=tickets)
+            assert S > 1 or not work.any(), "the sum must be zero again for the next step"
+            assert not tickets.any()
+        got[fused] = (out.float().clone(), kp.float().clone(), vp.float().clone())
+    torch.testing.assert_close(got[True][0], got[False][0], atol=2e-2, rtol=2e-2)
+    torch.testing.assert_close(got[True][1], got[False][1], atol=1e-2, rtol=8e-3)   # (x0*c - x1*s may contract differently: one ulp)
+    torch.testing.assert_close(got[True][2], got[False][2], atol=0, rtol=8e-3)
