@@ -15,6 +15,7 @@ not depend on which other requests share its batch.
 """
 from __future__ import annotations
 
+import struct
 from dataclasses import dataclass
 from typing import Optional, Sequence
 
@@ -63,9 +64,6 @@ def draw_on_device(logits: torch.Tensor, cfg: SamplerConfig, requests: torch.Ten
     ``requests`` and ``draws`` int32 [rows], ``recent`` int32 [rows, <= 64] with -1 for none (or ``None``).
     ``seed_dev``: the seed is read from device memory (a captured step); ``temperature``: the constant of
     :func:`temperature_rows`, made once by a caller that runs this many times."""
-    rows = logits.shape[0]
-    if temperature is None:
-        temperature = temperature_rows(cfg, rows, logits.device)
     if cfg.filtered:
         # every filter in one kernel of ours; top-k off (0, or at least the vocabulary) is a path of its own there
         top_k = cfg.top_k if 0 < cfg.top_k < logits.shape[1] else 0
@@ -76,9 +74,28 @@ def draw_on_device(logits: torch.Tensor, cfg: SamplerConfig, requests: torch.Ten
             # a small top-k: only what it can keep is looked at
             return K.filter_draw(logits, cfg.temperature, top_k, cfg.top_p, cfg.min_p, cfg.repetition_penalty, rec,
                                  requests, draws, seed, out, seed_dev)
-        work = K.filter_logits(logits, cfg.temperature, top_k, cfg.top_p, cfg.min_p, cfg.repetition_penalty, rec)
-        return K.sample(work, temperature, requests, draws, seed, out, seed_dev)
+        logits = K.filter_logits(logits, cfg.temperature, top_k, cfg.top_p, cfg.min_p, cfg.repetition_penalty, rec)
+    if temperature is None:
+        temperature = temperature_rows(cfg, logits.shape[0], logits.device)
     return K.sample(logits, temperature, requests, draws, seed, out, seed_dev)
+
+
+def _int32_rows(parts: Sequence[Sequence[int]], rows: Sequence[Sequence[int]], width: int, device: torch.device) -> torch.Tensor:
+    """``parts`` one after another, then the last ``width`` numbers of each of ``rows`` (-1 behind a shorter one), as
+    one int32 tensor on the device: one copy.  (64 rows of 64 tokens: 70 us of host time and one copy, against 310 us
+    for a tensor of nested lists.)"""
+    flat: list = []
+    for p in parts:
+        flat.extend(p)          # (+= would add an array's numbers to the list's)
+    for r in rows:
+        n = len(r)
+        flat.extend(r[n - width:] if n > width else r)
+        if n < width:
+            flat.extend([-1] * (width - n))
+    if not flat:
+        return torch.empty((0,), dtype=torch.int32, device=device)
+    host = torch.frombuffer(bytearray(struct.pack(f"{len(flat)}i", *flat)), dtype=torch.int32)
+    return host.to(device, non_blocking=True)
 
 
 class DeviceSampler:
@@ -93,10 +110,12 @@ class DeviceSampler:
         if cfg.greedy:
             return K.argmax(logits)
         dev = logits.device
-        meta = torch.tensor([list(requests), list(draws)], dtype=torch.int32).to(dev, non_blocking=True)
-        rec = None
+        rows, kept = len(requests), ()
+        if len(draws) != rows:
+            raise ValueError(f"{rows} requests, {len(draws)} draw indices")
         if cfg.filtered and recent is not None and cfg.repetition_penalty > 1.0:
-            width = min(RECENT_WINDOW, K.FILTER_MAX_RECENT)
-            rec = torch.tensor([(list(r)[-width:] + [-1] * width)[:width] for r in recent],
-                               dtype=torch.int32).to(dev, non_blocking=True)
-        return draw_on_device(logits, cfg, meta[0], meta[1], rec, self.seed)
+            kept = recent
+        width = min(RECENT_WINDOW, K.FILTER_MAX_RECENT)
+        ints = _int32_rows((requests, draws), kept, width, dev)
+        rec = ints[2 * rows:].view(len(kept), width) if len(kept) else None
+        return draw_on_device(logits, cfg, ints[:rows], ints[rows:2 * rows], rec, self.seed)
