@@ -1931,6 +1931,26 @@ def gemm_tc_workspace_floats(ra: int, rb: int, bn: int, splits: int) -> int:
     return ((ra + TC_TILE_M - 1) // TC_TILE_M) * ((rb + bn - 1) // bn) * splits * bn * TC_TILE_M
 
 
+def gemm_tc_stream(w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, epilogue: int) -> bool:
+    """The product of 1 to 128 tokens x[T, K] with a weight w[N, K] by persistent CTAs that stream the weight, in float32
+    [T, N]: ``TC_STORE_F32``, or ``TC_RED_F32`` added into ``out`` (order not fixed).  False where the output's alignment
+    rules it out (nothing ran)."""
+    for n, t in (("w", w), ("x", x)):
+        if not t.is_cuda or t.dtype != torch.bfloat16 or t.dim() != 2 or t.stride(1) != 1:
+            raise KernelError(f"gemm_tc_stream: {n} must be a 2-D bfloat16 GPU tensor with unit inner stride")
+    (n, k), (t, k2) = w.shape, x.shape
+    if k != k2:
+        raise KernelError(f"gemm_tc_stream: w has K={k}, x has K={k2}")
+    if out.dim() != 2 or tuple(out.shape) != (t, n) or out.stride(1) != 1 or out.dtype != torch.float32:
+        raise KernelError(f"gemm_tc_stream: out must be float32 [{t}, {n}] with unit inner stride")
+    st = _lib("gemm_tc").dlgo_gemm_tc_stream(_ptr(w), _i(n), _i(w.stride(0)), _ptr(x), _i(t), _i(x.stride(0)), _i(k), _ptr(out),
+                                             _i(out.stride(0)), _i(epilogue), _stream())
+    if st == -2:        # alignment
+        return False
+    _check(st, "gemm_tc_stream")
+    return True
+
+
 def gemm_tc(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, transposed: bool, epilogue: int, bn: int,
             splits: int = 1, workspace: Optional[torch.Tensor] = None,
             counters: Optional[torch.Tensor] = None, static_operand: int = 0, pair_tile: int = 0,

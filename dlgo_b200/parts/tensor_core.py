@@ -50,6 +50,9 @@ MIN_KBLOCKS_PER_SPLIT = int(os.environ.get("DLGO_TC_MIN_KBLOCKS", 3))   # (3 aga
 ORDERED_SUMS = os.environ.get("DLGO_ORDERED_SUMS", "0") == "1"
 RED_MAX_TOKENS = int(os.environ.get("DLGO_TC_RED_MAX_TOKENS", 64))
 
+# More than 16 tokens: weights of at least as many tiles per SM (the head) go through persistent CTAs (gemm_tc_stream).
+STREAM_MIN_TILES = int(os.environ.get("DLGO_TC_STREAM_MIN_TILES", 4))
+
 _workspaces: Dict[int, List[torch.Tensor]] = {}
 _counters: Dict[int, torch.Tensor] = {}
 
@@ -121,6 +124,8 @@ class TensorCorePlan:
                                   device=x.device)
         if t <= SKINNY_MAX:
             bn, splits = skinny_shape(t, self.n, self.k, self.weight.device, self.swiglu)
+            if bn > 16 and self._stream(x, epi, out):
+                return out
             if not ORDERED_SUMS and epi == K.TC_ADD_F32 and splits > 1 and t <= RED_MAX_TOKENS:
                 return K.gemm_tc(self.weight, x, out, True, K.TC_RED_F32, bn, splits, static_operand=1)
             ws = cnt = None
@@ -130,6 +135,12 @@ class TensorCorePlan:
             return K.gemm_tc(self.weight, x, out, True, epi, bn, splits, ws, cnt, static_operand=1, glu=self.clamp)
         bn, pair = self.many_token_shape(t)
         return K.gemm_tc(x, self.weight, out, False, epi, bn, static_operand=2, pair_tile=pair, glu=self.clamp)
+
+    def _stream(self, x, epi: int, out: torch.Tensor) -> bool:
+        """The product by the kernel that streams the weight through persistent CTAs, where it is the better one."""
+        if epi != K.TC_STORE_F32 or self.n < STREAM_MIN_TILES * K.TC_TILE_M * sm_count(x.device):
+            return False
+        return K.gemm_tc_stream(self.weight, x, out, epi)
 
     def bias_act(self, x, bias: Optional[torch.Tensor], act: int) -> torch.Tensor:
         """``act(x . W^T + bias)`` as bfloat16 [tokens, out], bias and activation in the contraction's epilogue

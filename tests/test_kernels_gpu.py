@@ -1124,3 +1124,26 @@ def test_decode_attention_in_even_shares_rotates_appends_and_clears(hq, hkv, hd,
     torch.testing.assert_close(got[True][0], got[False][0], atol=2e-2, rtol=2e-2)
     torch.testing.assert_close(got[True][1], got[False][1], atol=1e-2, rtol=8e-3)   # (x0*c - x1*s may contract differently: one ulp)
     torch.testing.assert_close(got[True][2], got[False][2], atol=0, rtol=8e-3)
+
+
+@pytest.mark.parametrize("T_", [1, 17, 32, 33, 64, 65, 128])
+@pytest.mark.parametrize("N,K_", [(128, 64), (160, 72), (2080, 520), (19200, 264), (28672, 1032)])
+def test_gemm_tc_stream(T_, N, K_):
+    """Runs that begin and end inside tiles and at their edges, rows and K that are no whole tiles.  fp32 sums of bfloat16
+    products (exact in fp32): 2^-24 of the absolute sum for each of K additions at most."""
+    k = K()
+    torch.manual_seed(N + T_)
+    x = torch.randn(T_, K_, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(N, K_, device=DEV) * 0.1).to(torch.bfloat16)
+    ref = x.double() @ w.double().t()
+    bound = (x.double().abs() @ w.double().abs().t()) * K_ * 2.0 ** -24
+    wide = torch.full((T_ + 1, N + 4), float("nan"), device=DEV)
+    assert k.gemm_tc_stream(w, x, wide[:T_, :N], k.TC_STORE_F32)
+    assert ((wide[:T_, :N].double() - ref).abs() <= bound).all()
+    assert torch.isnan(wide[T_]).all() and torch.isnan(wide[:, N:]).all()
+    assert not k.gemm_tc_stream(w, x, torch.empty(T_, N + 1, device=DEV)[:, :N], k.TC_STORE_F32)    # rows TMA cannot describe
+    acc = torch.randn(T_, N, device=DEV)
+    want = acc.double() + ref
+    assert k.gemm_tc_stream(w, x, acc, k.TC_RED_F32)
+    assert ((acc.double() - want).abs() <= bound + want.abs() * 2.0 ** -22 + 1e-6).all()
+    k.check_device_errors()
