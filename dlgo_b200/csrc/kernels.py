@@ -2466,7 +2466,7 @@ def decode_layers(desc: torch.Tensor, n_layers: int, residual: torch.Tensor, hid
 
 # ------------------------------------------------------------------ the layer loop of a prompt step, native
 class PromptEntryPoints(ctypes.Structure):
-    _fields_ = [(n, _p) for n in ("rmsnorm", "gemm_tc", "rope_append", "attention", "gemm_tc_rope")]
+    _fields_ = [(n, _p) for n in ("rmsnorm", "gemm_tc", "rope_append", "attention", "gemm_tc_rope", "gemm_tc_stream")]
 
 
 class PromptShape(ctypes.Structure):
@@ -2482,7 +2482,8 @@ class PromptLayer(ctypes.Structure):
 class PromptStep(ctypes.Structure):
     _fields_ = [("tokens", _i), ("residual", _p), ("x", _p), ("qkv", _p), ("attn_out", _p), ("h", _p), ("cos_t", _p),
                 ("sin_t", _p), ("token_pos", _p), ("token_seq", _p), ("seq_slot", _p), ("page_table", _p),
-                ("max_pages", _i), ("tiles", _p), ("n_tiles", _i), ("bn", _i * 4), ("pair", _i * 4), ("fuse_rope", _i)]
+                ("max_pages", _i), ("tiles", _p), ("n_tiles", _i), ("bn", _i * 4), ("pair", _i * 4), ("fuse_rope", _i),
+                ("form", _i * 4), ("splits", _i * 4), ("qkv_sum", _p)]
 
 
 PROMPT_CALLS = ("mixer norm", "q/k/v projection", "rotation and cache append (0 launches where the projection does it)", "attention", "output projection",
@@ -2497,7 +2498,7 @@ def prompt_entry_points() -> PromptEntryPoints:
     return PromptEntryPoints(address("elementwise", "dlgo_rmsnorm"), address("gemm_tc", "dlgo_gemm_tc"),
                              address("rope_append", "dlgo_rope_append"),
                              address("attention_prefill_tc", "dlgo_attention_prefill_tc"),
-                             address("gemm_tc", "dlgo_gemm_tc_rope"))
+                             address("gemm_tc", "dlgo_gemm_tc_rope"), address("gemm_tc", "dlgo_gemm_tc_stream"))
 
 
 def prompt_layers_describe(layers: Sequence[dict]) -> tuple:

@@ -47,6 +47,9 @@ struct DlgoRopeArgs {
 typedef int (*GemmTcRopeFn)(const void* x, int T, int ldx, const void* w, int Rb, int ldw, int K, void* qkv, int ldo,
                             int pair_tile, const DlgoRopeArgs* rope, cudaStream_t stream);
 
+typedef int (*GemmTcStreamFn)(const void* w, int N, int ldw, const void* x, int T, int ldx, int K, void* out, int ldo,
+                              int epilogue, cudaStream_t stream);
+
 // Entry points of the kernel libraries.
 struct DlgoPromptEntryPoints {
   RmsNormFn rmsnorm;
@@ -54,6 +57,7 @@ struct DlgoPromptEntryPoints {
   RopeAppendFn rope_append;
   AttentionFn attention;
   GemmTcRopeFn gemm_tc_rope;
+  GemmTcStreamFn gemm_tc_stream;
 };
 
 // What the layers of a run share.
@@ -99,12 +103,16 @@ struct DlgoPromptStep {
   int bn[4];              // tile width of qkv, o, gate_up, down
   int pair[4];            // their CTA-pair tile (0: none)
   int fuse_rope;          // the q/k/v projection's epilogue rotates and appends: no launch for that
+  int form[4];            // of each product: 0 many tokens (tokens are M), 1 few tokens (the weight is M, bn tokens a
+                          // tile, `splits` K-slices), 2 the weight streamed by persistent CTAs (added into fp32)
+  int splits[4];
+  float* qkv_sum;         // forms 1 and 2: [tokens, (heads + 2 kv_heads) * head_dim] fp32, zero; left zero
 };
 
 }  // extern "C"
 
 namespace {
-constexpr int TC_STORE = 0, TC_ADD_F32 = 2, TC_SWIGLU = 3;   // epilogue codes of dlgo_gemm_tc
+constexpr int TC_STORE = 0, TC_ADD_F32 = 2, TC_SWIGLU = 3, TC_RED_F32 = 5;   // epilogue codes of dlgo_gemm_tc
 }
 
 // Runs `n_layers` layers.  Returns 0, or the first non-zero status with *failed_call = 8 * layer + call
@@ -114,12 +122,21 @@ DLGO_EXPORT int dlgo_prompt_layers(const DlgoPromptEntryPoints* fn, const DlgoPr
                                    int* failed_call, cudaStream_t stream) {
   if (fn == nullptr || s == nullptr || layers == nullptr || p == nullptr) return DLGO_ERR_SIZE;
   if (fn->rmsnorm == nullptr || fn->gemm_tc == nullptr || fn->rope_append == nullptr || fn->attention == nullptr ||
-      fn->gemm_tc_rope == nullptr)
+      fn->gemm_tc_rope == nullptr || fn->gemm_tc_stream == nullptr)
     return DLGO_ERR_DRIVER;
   const int T = p->tokens, d = s->hidden;
   const int q_dim = s->heads * s->head_dim, n_cols = (s->heads + 2 * s->kv_heads) * s->head_dim;
   if (T <= 0 || n_layers <= 0) return DLGO_OK;
   int st = DLGO_OK, call = 0;
+  // product j of a layer: x[T, K] with w[N, K] into out (row stride ldo)
+  auto product = [&](int j, const void* x, const void* w, int N, int K, void* out, int ldo, int epilogue) {
+    if (p->form[j] == 2)
+      return epilogue == TC_ADD_F32 ? fn->gemm_tc_stream(w, N, K, x, T, K, K, out, ldo, TC_RED_F32, stream) : DLGO_ERR_SIZE;
+    if (p->form[j] == 1)
+      return fn->gemm_tc(w, N, K, x, T, K, K, out, ldo, 1, epilogue == TC_ADD_F32 && p->splits[j] > 1 ? TC_RED_F32 : epilogue,
+                         p->bn[j], p->splits[j], nullptr, nullptr, 1, 0, stream);
+    return fn->gemm_tc(x, T, K, w, N, K, K, out, ldo, 0, epilogue, p->bn[j], 1, nullptr, nullptr, 2, p->pair[j], stream);
+  };
 #define DLGO_STEP(expr)                           \
   do {                                            \
     st = (expr);                                  \
@@ -139,23 +156,21 @@ DLGO_EXPORT int dlgo_prompt_layers(const DlgoPromptEntryPoints* fn, const DlgoPr
       DLGO_STEP(fn->gemm_tc_rope(p->x, T, d, L.w_qkv, n_cols, d, d, p->qkv, n_cols, p->pair[0], &rope, stream));
       ++call;
     } else {
-      DLGO_STEP(fn->gemm_tc(p->x, T, d, L.w_qkv, n_cols, d, d, p->qkv, n_cols, 0, TC_STORE, p->bn[0], 1, nullptr,
-                            nullptr, 2, p->pair[0], stream));
+      const bool sum = p->form[0] != 0;       // K-slices meet in one fp32 sum, which the rotation reads and clears
+      if (sum && p->qkv_sum == nullptr) return DLGO_ERR_SIZE;
+      DLGO_STEP(product(0, p->x, L.w_qkv, n_cols, d, sum ? (void*)p->qkv_sum : p->qkv, n_cols, sum ? TC_ADD_F32 : TC_STORE));
       DLGO_STEP(fn->rope_append(p->qkv, DLGO_BF16, T, n_cols, p->cos_t, p->sin_t, p->token_pos, p->token_seq,
                                 p->seq_slot, p->page_table, p->max_pages, L.kpages, L.vpages, s->heads, s->kv_heads,
-                                s->head_dim, s->rotary_dim, s->page_size, s->interleaved, L.write_cache, nullptr, 0, 0,
-                                0, stream));
+                                s->head_dim, s->rotary_dim, s->page_size, s->interleaved, L.write_cache,
+                                sum ? p->qkv_sum : nullptr, sum ? 1 : 0, 0, sum ? 1 : 0, stream));
     }
     DLGO_STEP(fn->attention(p->qkv, T, n_cols, L.kpages, L.vpages, L.n_pages, p->page_table, p->max_pages, p->tiles,
                             p->n_tiles, p->seq_slot, p->token_pos, p->attn_out, q_dim, s->heads, s->kv_heads,
                             s->head_dim, s->window, s->scale, nullptr, 0, stream));
-    DLGO_STEP(fn->gemm_tc(p->attn_out, T, q_dim, L.w_o, d, q_dim, q_dim, p->residual, d, 0, TC_ADD_F32, p->bn[1], 1,
-                          nullptr, nullptr, 2, p->pair[1], stream));
+    DLGO_STEP(product(1, p->attn_out, L.w_o, d, q_dim, p->residual, d, TC_ADD_F32));
     DLGO_STEP(fn->rmsnorm(p->residual, L.norm2_w, p->x, DLGO_BF16, nullptr, T, d, L.eps2, stream));
-    DLGO_STEP(fn->gemm_tc(p->x, T, d, L.w_gate_up, 2 * s->ffn, d, d, p->h, s->ffn, 0, TC_SWIGLU, p->bn[2], 1, nullptr,
-                          nullptr, 2, p->pair[2], stream));
-    DLGO_STEP(fn->gemm_tc(p->h, T, s->ffn, L.w_down, d, s->ffn, s->ffn, p->residual, d, 0, TC_ADD_F32, p->bn[3], 1,
-                          nullptr, nullptr, 2, p->pair[3], stream));
+    DLGO_STEP(product(2, p->x, L.w_gate_up, 2 * s->ffn, d, p->h, s->ffn, TC_SWIGLU));
+    DLGO_STEP(product(3, p->h, L.w_down, d, s->ffn, p->residual, d, TC_ADD_F32));
   }
 #undef DLGO_STEP
   return DLGO_OK;

@@ -10,7 +10,8 @@ calls the same entry points with the same arguments from
 sizes, constants, tensors and tile shapes from the parts the model was built
 from, launches what they launch, and steps aside (the parts run one by one) for
 anything else: other blocks, mixers, feed-forwards or norms, float32, head
-sizes the tensor-core attention does not take, few tokens, per-kernel timing.
+sizes the tensor-core attention does not take, per-kernel timing; with
+``DLGO_ORDERED_SUMS`` also for few tokens.
 
 ``DLGO_NATIVE_PROMPT=0`` switches it off.
 """
@@ -30,6 +31,15 @@ from ..parts.feedforward import SwiGLU
 from ..parts.norm import RMSNorm
 from ..parts.rope import RotaryEmbedding
 
+# Which products a prompt step takes, by its tokens.  Up to 64: those of a decode step (the weight is the tensor core's M
+# operand).  Up to STREAM_MAX: q|k|v, output and down projection added into fp32 by CTAs that stream the weight
+# (gemm_tc_stream), gate/up by tiles of 256 tokens; above, such tiles are half full at least and all products take them.
+# Measured on a B200, Llama 3.2 1B sizes, us a prompt: 8 tokens 800, 64 tokens 965 (issued part by part from Python: 2,250
+# whatever the length up to 64); 80 tokens 1,285 and 117 1,323 (tiles of 256 tokens for all products: 1,436 and 1,444); 3.1
+# 8B sizes, 30 tokens 3,685 (4,268), 100 tokens 4,470 (4,815).  In 117 tokens the down projection takes 11.3 us against
+# 13.3, q|k|v with the rotation's launch 14 against 20, whose 12 tiles leave most SMs idle; gate/up would take 27
+# against 21.
+STREAM_MAX = int(os.environ.get("DLGO_PROMPT_STREAM_MAX", 128))
 ENABLED = os.environ.get("DLGO_NATIVE_PROMPT", "1") != "0"
 
 
@@ -68,7 +78,9 @@ class PromptRun:
     def takes(self, ctx: Any, cache: Any) -> bool:
         hd = self.sig[3]
         view = cache.view(self.first)
-        return (not ctx.decode and ctx.n_tokens > tensor_core.SKINNY_MAX and view is not None and
+        few = ctx.n_tokens <= tensor_core.SKINNY_MAX     # (their K-slices meet in no fixed order)
+        return (not ctx.decode and view is not None and
+                (not few or not (tensor_core.ORDERED_SUMS or ctx.n_tokens > tensor_core.RED_MAX_TOKENS)) and
                 K._profile_events is None and
                 K.attention_prefill_tc_takes(torch.bfloat16, hd, view.page_size) and view.keys.dtype == torch.bfloat16)
 
@@ -119,8 +131,19 @@ class PromptRun:
         step.max_pages = view.page_table.shape[1]
         step.tiles, step.n_tiles = tiles.data_ptr(), n_tiles
         for j, lin in enumerate((blk.mixer.wqkv, blk.mixer.wo, blk.ffn.w_gate_up, blk.ffn.w_down)):
-            step.bn[j], step.pair[j] = lin._tc.many_token_shape(T)
-        step.fuse_rope = 1 if (pe_name is not None and blk.mixer.fuses_prompt_rope(ctx, view, model.positions)) else 0
+            swiglu = j == 2
+            if T <= tensor_core.SKINNY_MAX:
+                step.form[j] = 1
+                step.bn[j], splits = tensor_core.skinny_shape(T, lin._tc.n, lin._tc.k, residual.device, swiglu)
+                step.splits[j] = 1 if swiglu else splits
+            else:
+                step.bn[j], step.pair[j] = lin._tc.many_token_shape(T)
+                if T <= STREAM_MAX and not swiglu and not tensor_core.ORDERED_SUMS and \
+                        "DLGO_TC_DIRECT_EPILOGUE" not in os.environ:
+                    step.form[j] = 2
+        if step.form[0] != 0:
+            step.qkv_sum = ctx.zeros(f"qkv_sum{n_cols}", T * n_cols, torch.float32).data_ptr()
+        step.fuse_rope = 1 if step.form[0] == 0 and pe_name is not None and blk.mixer.fuses_prompt_rope(ctx, view, model.positions) else 0
         shape = K.PromptShape(d, hq, hkv, hd, f, rot, 1 if inter else 0, window, view.page_size, scale)
         K.prompt_layers(self._entry, shape, layers, step)
 

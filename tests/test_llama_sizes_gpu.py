@@ -176,6 +176,37 @@ def test_prompt_steps_run_through_the_native_layer_loop_and_match_the_parts(big,
     assert eng32.model.prompt_runs == {} and prompt_run.ENABLED
 
 
+@pytest.mark.parametrize("lens", [[2], [5, 9], [17], [30, 3, 31], [65], [50, 27], [128]])
+def test_short_prompt_steps_through_the_native_layer_loop_match_the_parts(big, lens, monkeypatch):
+    """Up to 64 tokens, up to 128: other products than longer prompts (the weight is the tensor core's M operand and its
+    K-slices meet in fp32), onto an empty cache and onto one that is not."""
+    from dlgo_b200.csrc import kernels
+    from dlgo_b200.engine.engine import Engine
+    d, _, _ = big
+    g = torch.Generator().manual_seed(sum(lens))
+    prompts, more = ([torch.randint(0, CFG["vocab_size"], (n,), generator=g).tolist() for n in lens] for _ in range(2))
+    calls = []
+    real = kernels.prompt_layers
+    monkeypatch.setattr(kernels, "prompt_layers", lambda e, sh, layers, step: (calls.append(step.tokens),
+                                                                                 real(e, sh, layers, step))[1])
+
+    def logits(eng):
+        slots = [eng.take_slot() for _ in prompts]
+        out = [eng.step(slots, p, [[len(q) - 1, 0] for q in p]).float().cpu() for p in (prompts, more)]
+        for s in slots:
+            eng.free_slot(s)
+        return torch.cat(out)
+
+    eng = Engine(d, dtype="bfloat16", max_tokens=1024, max_seq_len=512)
+    got = logits(eng)
+    assert calls == [sum(lens)] * 2
+    monkeypatch.setattr(eng.model, "prompt_runs", {})
+    want = logits(eng)
+    assert len(calls) == 2
+    assert float((got - want).abs().max()) <= 3e-2 * float(want.abs().max())     # (sums in no fixed order: bfloat16 rounding)
+    kernels.check_device_errors()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_llama_8b_layer_sizes_against_the_plain_implementation(big8, dtype):
     from dlgo_b200.engine.engine import Engine
