@@ -68,28 +68,26 @@ __device__ __forceinline__ void finish(void* out, size_t at, float v) {
 // ------------------------------------------------------------------ many rows
 // Bound by the fp32 pipes and, as closely, by what shared memory delivers to registers (128 bytes a clock, broadcast or
 // not): 8 x 8 outputs per thread need 16 words of 16 bytes for 128 packed multiply-adds, 64 clocks of either.  A warp
-// takes 64 x 32 outputs, a block 64 WM x 64; the four quarters of K are the blocks of a cluster (as many as are not
-// empty), which evens out the last wave, and meet through distributed shared memory.  A thread's pairs take 128
-// registers; the sum over a quarter's spans waits in shared memory, a slot per output and thread.
-// Rows lie in a ring of four stages of 16 k, 20 floats apart: the rows that a quarter warp reads are on different banks.
-// Measured on a B200 (TFLOP/s; 64 x 64 outputs of scalar multiply-adds with a synchronous load of every 16 k before):
-// 366 x 16384 x 2048 38 (4), 366 x 2048 x 8192 35; scalar multiply-adds in this layout 27; 8 x 4 outputs per thread with
-// twelve warps an SM 36 and, without the cluster, 20.  The fp32 pipes give 74 at most.
-constexpr int BN = 64, KSTEP = 16, ROW = KSTEP + 4, STAGES = 4;
-template <int WM> struct TileShape {
-  static constexpr int BM = 64 * WM, THREADS = 64 * WM;
-  static constexpr int RING = STAGES * (BM + BN) * ROW;      // floats
-  static constexpr int SMEM = (RING + BM * BN) * 4;
-};
+// takes 64 x 32 outputs, a block of two warps 64 x 64, four blocks an SM; the four quarters of K are the blocks of a
+// cluster (as many as are not empty), which evens out the last wave, and meet through distributed shared memory.  A
+// thread's pairs take 128 registers; the sum over a quarter's spans waits in shared memory, a slot per output and thread.
+// Rows lie in a ring of three stages of 16 k, 20 floats apart: the rows that a quarter warp reads are on different banks.
+// Measured on a B200 (TFLOP/s): 567 x 16384 x 2048 41, 567 x 2048 x 8192 35, 64 x 16384 x 2048 34.  Blocks of 128 x 64 with
+// four warps and four stages, two an SM, have as many warps there and more padding: 36, 34 and 19.  64 x 64 outputs of
+// scalar multiply-adds with a synchronous load of every 16 k (before) 4; scalar multiply-adds in this layout 29 where
+// packed ones give 38; 8 x 4 outputs per thread with twelve warps an SM and no cluster 36 and 20 for 366 rows.  The order
+// of the multiply-adds and the width of the loads from shared memory change less than 2 %.  The fp32 pipes give 74 at most.
+constexpr int BM = 64, BN = 64, KSTEP = 16, ROW = KSTEP + 4, STAGES = 3, THREADS = 64;
+constexpr int TILE_RING = STAGES * (BM + BN) * ROW;      // floats
+constexpr int TILE_SMEM = (TILE_RING + BM * BN) * 4;
 
-template <typename T, int EPI, int WM, bool VEC>
-__global__ void __launch_bounds__(64 * WM, WM == 2 ? 2 : 3)
+template <typename T, int EPI, bool VEC>
+__global__ void __launch_bounds__(THREADS, 4)
 gemm_simt_tile_kernel(const T* A, const T* __restrict__ W, void* out, int M, int N, int K, int lda, int ldw, int ldo) {
   namespace cg = cooperative_groups;
-  using S = TileShape<WM>;
-  constexpr int BM = S::BM, THREADS = S::THREADS, LROWS = THREADS / 4;
+  constexpr int LROWS = THREADS / 4;
   extern __shared__ __align__(16) float ring[];
-  float4* sums = reinterpret_cast<float4*>(ring + S::RING);   // [16][THREADS]: of thread t's output row i, columns 4 h .. 4 h + 3 at 2 i + h
+  float4* sums = reinterpret_cast<float4*>(ring + TILE_RING);   // [16][THREADS]: of thread t's output row i, columns 4 h .. 4 h + 3 at 2 i + h
   pdl_launch_dependents();
   cg::cluster_group cl = cg::this_cluster();
   const int quarters = (int)cl.num_blocks(), quarter = (int)cl.block_rank();
@@ -97,8 +95,8 @@ gemm_simt_tile_kernel(const T* A, const T* __restrict__ W, void* out, int M, int
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m_tiles = (M + BM - 1) / BM;                      // blocks of the same weight rows follow one another
   const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
-  const int tm = (warp >> 1) * 64 + (lane >> 2);              // rows tm + 8 i
-  const int tn = (warp & 1) * 32 + (lane & 3) * 2;            // columns tn + (j & 1) + 8 (j >> 1)
+  const int tm = lane >> 2;                                   // rows tm + 8 i
+  const int tn = warp * 32 + (lane & 3) * 2;                  // columns tn + (j & 1) + 8 (j >> 1)
   const int lrow = tid >> 2, lk = (tid & 3) * 4;              // loading
   const int span = span_length(K);
   const int k_begin = quarter * QUARTER * span, k_end = min(K, k_begin + QUARTER * span);
@@ -159,7 +157,10 @@ gemm_simt_tile_kernel(const T* A, const T* __restrict__ W, void* out, int M, int
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) fma_two(acc[i][j], a[now][i], b[now][j]);
+        for (int jj = 0; jj < 8; ++jj) {
+          const int j = (i & 1) ? 7 - jj : jj;          // (a row after another shares an operand at the turn)
+          fma_two(acc[i][j], a[now][i], b[now][j]);
+        }
     }
     if (++in_span == span_steps || s == steps - 1) {
 #pragma unroll
@@ -354,19 +355,18 @@ int launch_few(const T* a, const T* w, void* out, int M, int N, int K, int lda, 
   return launch_status();
 }
 
-template <typename T, int EPI, int WM, bool VEC>
+template <typename T, int EPI, bool VEC>
 int launch_tile(const T* a, const T* w, void* out, int M, int N, int K, int lda, int ldw, int ldo, cudaStream_t stream) {
-  using S = TileShape<WM>;
   const int quarter = QUARTER * span_length(K), quarters = (K + quarter - 1) / quarter;
-  const long long m_tiles = (M + S::BM - 1) / S::BM, n_tiles = (N + BN - 1) / BN;
+  const long long m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
   if (M > 65535 * 64 || m_tiles * n_tiles * quarters > 0x7fffffffLL) return DLGO_ERR_SIZE;
-  allow_smem(gemm_simt_tile_kernel<T, EPI, WM, VEC>, S::SMEM);
-  launch_kernel_cluster(gemm_simt_tile_kernel<T, EPI, WM, VEC>, dim3((unsigned)(m_tiles * n_tiles * quarters)), dim3(S::THREADS),
-                        S::SMEM, stream, dim3(quarters, 1, 1), a, w, out, M, N, K, lda, ldw, ldo);
+  allow_smem(gemm_simt_tile_kernel<T, EPI, VEC>, TILE_SMEM);
+  launch_kernel_cluster(gemm_simt_tile_kernel<T, EPI, VEC>, dim3((unsigned)(m_tiles * n_tiles * quarters)), dim3(THREADS),
+                        TILE_SMEM, stream, dim3(quarters, 1, 1), a, w, out, M, N, K, lda, ldw, ldo);
   return launch_status();
 }
 
-// Rows up to which the few-row kernel runs: at 16 rows of 16384 x 2048 it takes 52 us and the tile kernel 128 us, which
+// Rows up to which the few-row kernel runs: at 16 rows of 16384 x 2048 it takes 52 us and the tile kernel 125 us, which
 // it takes for 17 to 64 rows alike.
 constexpr int FEW_MAX = 16;
 
@@ -381,9 +381,7 @@ int launch_gemm_simt(const T* a, const T* w, void* out, int M, int N, int K, int
     if (M <= 8) return launch_few<T, EPI, 8, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
     return launch_few<T, EPI, 16, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
   }
-  // 64 rows a block where 128 would leave half of the only or second block empty
-  return M <= 64 || (M > 128 && M <= 192) ? launch_tile<T, EPI, 1, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream)
-                                          : launch_tile<T, EPI, 2, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
+  return launch_tile<T, EPI, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
 }
 
 template <typename T, bool VEC>
