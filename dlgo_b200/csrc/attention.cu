@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(AttnParams p) {
   constexpr int VN = Vec<T>::N;
   const int vec_per_row = hd / VN;
   for (int pg = pg_b; pg < pg_e; ++pg) {
-    const int page = p.page_table[(size_t)slot * p.max_pages + pg];
+    const int page = readable_page(p.page_table + (size_t)slot * p.max_pages, pg);
     const size_t base = ((size_t)page * p.Hkv + kvh) * PS * hd;
     const T* kp = (const T*)p.kpages + base;
     const T* vp = (const T*)p.vpages + base;

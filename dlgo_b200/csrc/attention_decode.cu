@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 4) attention_decode_kernel(DecPar
     const int pg = pg_b + tile / tiles_per_page;
     const int key0 = (tile % tiles_per_page) * TILE;
     if (pg * PS + key0 >= t_end) continue;
-    const int page = p.page_table[(size_t)slot * p.max_pages + pg];
+    const int page = readable_page(p.page_table + (size_t)slot * p.max_pages, pg);
     const size_t base = (((size_t)page * p.Hkv + kvh) * PS + key0) * HD;
     const char* kp = (const char*)((const T*)p.kpages + base);
     const char* vp = (const char*)((const T*)p.vpages + base);
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 4) attention_decode_kernel(DecPar
     const int pg = pg_b + tile / tiles_per_page;
     const int key0 = (tile % tiles_per_page) * TILE;
     if (pg * PS + key0 >= t_end) continue;                       // wholly beyond the sequence (warp-uniform)
-    const int page = p.page_table[(size_t)slot * p.max_pages + pg];
+    const int page = readable_page(p.page_table + (size_t)slot * p.max_pages, pg);
     const size_t base = ((size_t)page * p.Hkv + kvh) * PS * HD;
     const T* kp = (const T*)p.kpages + base;
     const T* vp = (const T*)p.vpages + base;

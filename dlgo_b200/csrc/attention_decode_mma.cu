@@ -37,6 +37,10 @@ constexpr int DM_THREADS = 128;
 constexpr int DM_WARPS = DM_THREADS / 32;
 constexpr int DM_GM = 8;   // query heads of a kv head per block
 
+// Set when a token's position had no page in the table (-1): the append is skipped, and the host reads the word
+// (dlgo_attention_decode_mma_error).
+__device__ int g_decode_append_error = 0;
+
 struct DecMmaParams {
   const __nv_bfloat16* q;
   int ldq;
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(DM_THREADS, HD <= 64 ? 4 : 2) attention_decode
     const int pg = pg_b + tile / tiles_per_page;
     const int key0 = (tile % tiles_per_page) * TK;
     if (pg * PS + key0 >= t_end) continue;
-    const int page = p.page_table[(size_t)slot * p.max_pages + pg];
+    const int page = readable_page(p.page_table + (size_t)slot * p.max_pages, pg);
     const size_t base = (((size_t)page * p.Hkv + kvh) * PS + key0) * HD;
     constexpr int LINES = TK * HD * 2 / 128;
     // (only for short slices, at most four rounds a warp: measured on a B200, hinting a long slice all
@@ -156,7 +160,8 @@ __global__ void __launch_bounds__(DM_THREADS, HD <= 64 ? 4 : 2) attention_decode
         const size_t row = (((size_t)page * p.Hkv + kvh) * PS + (pos % PS)) * HD;
         const float* kin = p.parts + (size_t)b * p.ldq + (size_t)(p.Hq + kvh) * HD;
         const float* vin = p.parts + (size_t)b * p.ldq + (size_t)(p.Hq + p.Hkv + kvh) * HD;
-        for (int i = lane; i < RH; i += 32) {
+        if (page < 0 && lane == 0) atomicExch(&g_decode_append_error, 1);   // never reserved: nothing is written
+        for (int i = lane; page >= 0 && i < RH; i += 32) {
           float k0 = 0.f, k1 = 0.f, v0 = 0.f, v1 = 0.f;
           for (int sl = 0; sl < p.S; ++sl) {          // slice order
             const size_t so = (size_t)sl * p.part_stride;
@@ -364,8 +369,6 @@ __global__ void __launch_bounds__(DM_THREADS, HD <= 64 ? 4 : 2) attention_decode
 constexpr int DS_SEGS = 4;
 constexpr int DS_MIN_TILES = 8;       // a block's least run: two tiles a warp
 constexpr int DS_MAX_B = 2048;        // sequences (their first tiles lie in shared memory)
-
-__device__ int g_decode_append_error = 0;
 
 template <int HD> constexpr size_t shares_smem(int B, int gm) {
   return (size_t)(B + 4) / 4 * 16 + (size_t)DS_SEGS * gm * HD * 2 + (size_t)DS_SEGS * DM_WARPS * gm * (HD + 4 + 2) * 4;
@@ -721,8 +724,7 @@ DLGO_EXPORT int dlgo_attention_decode_mma_takes(int hd, int page_size, int n_spl
   return (hd == 64 || hd == 128) && page_size % 32 == 0 && n_splits >= 1 && n_splits <= 65535;
 }
 
-// 1 if an append of a launch of even shares was skipped since the last call because its position had no page (clears the
-// word).
+// 1 if an append was skipped since the last call because its position had no page (clears the word).
 DLGO_EXPORT int dlgo_attention_decode_mma_error() {
   int v = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_decode_append_error, sizeof(int)) != cudaSuccess) return -1;

@@ -7,6 +7,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace dlgo {
 
 // d (rows 0-7 only) += A (rows 0-7; rows 8-15 are zero) * B
@@ -69,7 +71,7 @@ __device__ __forceinline__ void decode_attend_tiles(const __nv_bfloat16* kpages,
     const int pg = pg_b + tile / tiles_per_page;
     const int key0 = (tile % tiles_per_page) * TK;
     if (pg * PS + key0 >= t_end) continue;                       // wholly beyond the sequence (warp-uniform)
-    const int page = page_row[pg];
+    const int page = readable_page(page_row, pg);
     const size_t base = ((size_t)page * Hkv + kvh) * PS * HD;
     const T* kp = kpages + base;
     const T* vp = vpages + base;

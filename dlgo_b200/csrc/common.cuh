@@ -148,6 +148,11 @@ inline void launch_kernel_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// The page of a sequence's keys and values that an attention kernel reads.  A live position without a page (-1 in the
+// table) has been reported by the kernel that should have stored it (an error word; the step's results are void); reading
+// in front of the cache would fault before anyone sees the word, so the cache's first page stands in.
+__device__ __forceinline__ int readable_page(const int* page_row, int pg) { return max(page_row[pg], 0); }
+
 // Diagnostic build (-DDLGO_TIMING): kernels stamp the global timer at named points, per block, and
 // the library exports dlgo_times() to fetch the stamps (8 per block, the first 1024 blocks).
 #ifdef DLGO_TIMING

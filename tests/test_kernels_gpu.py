@@ -1147,3 +1147,58 @@ def test_gemm_tc_stream(T_, N, K_):
     assert k.gemm_tc_stream(w, x, acc, k.TC_RED_F32)
     assert ((acc.double() - want).abs() <= bound + want.abs() * 2.0 ** -22 + 1e-6).all()
     k.check_device_errors()
+
+
+@pytest.mark.parametrize("kernel", ["general", "decode", "mma", "mma cluster", "mma shares", "mma fused", "mma fused shares"])
+@pytest.mark.parametrize("hd", [64, 128])
+def test_a_live_position_without_a_page_is_not_written_and_not_read_in_front_of_the_cache(kernel, hd):
+    """Sequence 1's newest position has no page.  Kernels that append say so and leave the cache alone; none reads at page
+    -1 (the first page stands in, whose keys and values come back); the other sequences are not touched."""
+    k = K()
+    hq, hkv, lens = 4, 2, [100, 65, 30]
+    B, ld = 3, (4 + 2 * 2) * hd
+    torch.manual_seed(hd)
+    q = (torch.randn(1, B, ld, device=DEV) * 0.6).to(torch.bfloat16)
+    pages = [torch.randn(6, hkv, 64, hd, device=DEV).to(torch.bfloat16) for _ in range(2)]
+    pt = torch.tensor([[1, 2], [3, 4], [5, -1]], dtype=torch.int32, device=DEV)
+    missing = torch.tensor([[1, 2], [3, -1], [5, -1]], dtype=torch.int32, device=DEV)
+    stand_in = torch.tensor([[1, 2], [3, 0], [5, -1]], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV)
+    seq = torch.arange(B, dtype=torch.int32, device=DEV)
+    cos, sin = torch.ones(128, hd // 2, device=DEV), torch.zeros(128, hd // 2, device=DEV)      # (no rotation)
+    fused = "fused" in kernel
+
+    def attend(table):
+        kp, vp = (x.clone() for x in pages)
+        out = torch.full((B, hq * hd), float("nan"), device=DEV, dtype=torch.bfloat16)
+        args = (hq, hkv, hd, hd ** -0.5, 0)
+        if kernel == "general":
+            gchunk = k.attention_tile_shape(hd, hq // hkv, True)[1]
+            tiles = torch.tensor([[i, i, 1] for i in range(B)], dtype=torch.int32, device=DEV)
+            k.attention(q[0], ld, B, kp, vp, table, tiles, 1, seq, pos, out, *args, 1, gchunk, None)
+        elif kernel == "decode":
+            k.attention_decode(q[0], ld, B, kp, vp, table, seq, pos, out, *args, 2, None, None)
+        else:
+            n = 0 if "shares" in kernel else (2 if "cluster" in kernel else 1)
+            scratch = torch.empty(k.attention_decode_shares_scratch(hq, hkv, hd), device=DEV)
+            tickets = torch.zeros(B * hkv, dtype=torch.int32, device=DEV)
+            if fused:
+                k.attention_decode_mma(None, ld, B, kp, vp, table, seq, pos, out, *args, n, 32, scratch, q.float(), cos, sin,
+                                       True, tickets=tickets)
+            else:
+                k.attention_decode_mma(q[0], ld, B, kp, vp, table, seq, pos, out, *args, n, 32, scratch, tickets=tickets)
+        return out, kp, vp
+
+    k.check_device_errors()
+    want, wk, wv = attend(pt)
+    k.check_device_errors()
+    got, gk, gv = attend(missing)
+    if fused:
+        with pytest.raises(k.KernelError):
+            k.check_device_errors()
+        wk[4], wv[4] = pages[0][4], pages[1][4]                 # what was not stored
+    k.check_device_errors()                                     # (the word is cleared by the read)
+    assert torch.equal(gk, wk) and torch.equal(gv, wv)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[2], want[2])
+    if not fused:
+        assert torch.equal(got[1], attend(stand_in)[0][1])
