@@ -88,13 +88,18 @@ def _int32_rows(parts: Sequence[Sequence[int]], rows: Sequence[Sequence[int]], w
     for p in parts:
         flat.extend(p)          # (+= would add an array's numbers to the list's)
     for r in rows:
+        if not isinstance(r, (list, tuple)):
+            r = list(r)         # (a deque cannot be sliced, an iterator has no length)
         n = len(r)
         flat.extend(r[n - width:] if n > width else r)
         if n < width:
             flat.extend([-1] * (width - n))
     if not flat:
         return torch.empty((0,), dtype=torch.int32, device=device)
-    host = torch.frombuffer(bytearray(struct.pack(f"{len(flat)}i", *flat)), dtype=torch.int32)
+    try:
+        host = torch.frombuffer(bytearray(struct.pack(f"{len(flat)}i", *flat)), dtype=torch.int32)
+    except struct.error:        # not whole numbers of 32 bits: a tensor's own conversion takes them, or says why not
+        host = torch.tensor(flat, dtype=torch.int32)
     return host.to(device, non_blocking=True)
 
 
@@ -110,11 +115,14 @@ class DeviceSampler:
         if cfg.greedy:
             return K.argmax(logits)
         dev = logits.device
-        rows, kept = len(requests), ()
+        requests, draws, kept = list(requests), list(draws), []
+        rows = len(requests)
         if len(draws) != rows:
             raise ValueError(f"{rows} requests, {len(draws)} draw indices")
         if cfg.filtered and recent is not None and cfg.repetition_penalty > 1.0:
-            kept = recent
+            kept = list(recent)
+            if not kept:
+                raise IndexError("recent tokens: a row of them for each row of logits, or None")
         width = min(RECENT_WINDOW, K.FILTER_MAX_RECENT)
         ints = _int32_rows((requests, draws), kept, width, dev)
         rec = ints[2 * rows:].view(len(kept), width) if len(kept) else None

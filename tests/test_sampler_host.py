@@ -1,9 +1,11 @@
 """What the device sampler copies to the GPU in one piece: requests, draw indices and windows of recent tokens."""
+from collections import deque
+
 import numpy as np
 import pytest
 import torch
 
-from dlgo_b200.sampling.sampler import _int32_rows
+from dlgo_b200.sampling.sampler import DeviceSampler, SamplerConfig, _int32_rows
 
 
 @pytest.mark.parametrize("kind", [list, tuple, np.array])
@@ -14,3 +16,35 @@ def test_rows_keep_their_last_tokens_and_are_padded(kind, lengths):
     got = _int32_rows((kind([5, 6]), kind([2 ** 31 - 1, 0])), [kind(r) for r in rows], width, torch.device("cpu"))
     want = [5, 6, 2 ** 31 - 1, 0] + [t for r in rows for t in (r[-width:] + [-1] * width)[:width]]
     assert got.dtype == torch.int32 and got.tolist() == want
+
+
+@pytest.mark.parametrize("kind", [deque, iter, torch.tensor, lambda r: [float(t) for t in r], lambda r: range(r[0], r[0] + len(r))])
+@pytest.mark.parametrize("n", [3, 64, 65, 200])
+def test_whatever_a_list_can_be_made_of_is_a_row(kind, n):
+    row = list(range(7, 7 + n))
+    got = _int32_rows((kind([5, 6]),), [kind(row), row], 64, torch.device("cpu"))
+    one = (row[-64:] + [-1] * 64)[:64]
+    assert got.dtype == torch.int32 and got.tolist() == [5, 6] + one + one
+
+
+@pytest.mark.parametrize("many", [2 ** 31, -2 ** 31 - 1])
+def test_numbers_beyond_32_bits_are_refused_as_a_tensor_refuses_them(many):
+    with pytest.raises(RuntimeError):
+        _int32_rows(([many], [0]), [], 64, torch.device("cpu"))
+
+
+def test_the_sampler_takes_iterators_and_deques_and_refuses_no_rows(monkeypatch):
+    from dlgo_b200.sampling import sampler as S
+    seen = []
+    monkeypatch.setattr(S, "draw_on_device", lambda logits, cfg, req, draws, rec, seed: seen.append((req, draws, rec)))
+    logits, cfg = torch.zeros(2, 300), SamplerConfig()
+    rows = [list(range(100)), [3, 4]]
+    for how in (lambda r: r, deque, iter):
+        DeviceSampler().sample(logits, cfg, how([8, 9]), how([1, 2]), how([how(r) for r in rows]))
+        req, draws, rec = seen.pop()
+        assert req.tolist() == [8, 9] and draws.tolist() == [1, 2]
+        assert rec.tolist() == [rows[0][-64:], rows[1] + [-1] * 62]
+    with pytest.raises(IndexError):
+        DeviceSampler().sample(logits, cfg, [8, 9], [1, 2], [])
+    with pytest.raises(ValueError):
+        DeviceSampler().sample(logits, cfg, [8, 9], [1], rows)
