@@ -1931,6 +1931,9 @@ def gemm_tc_workspace_floats(ra: int, rb: int, bn: int, splits: int) -> int:
     return ((ra + TC_TILE_M - 1) // TC_TILE_M) * ((rb + bn - 1) // bn) * splits * bn * TC_TILE_M
 
 
+GEMM_TC_STREAM_MAX = 128      # tokens that gemm_tc_stream takes
+
+
 def gemm_tc_stream(w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, epilogue: int) -> bool:
     """The product of 1 to 128 tokens x[T, K] with a weight w[N, K] by persistent CTAs that stream the weight, in float32
     [T, N]: ``TC_STORE_F32``, or ``TC_RED_F32`` added into ``out`` (order not fixed).  False where the output's alignment

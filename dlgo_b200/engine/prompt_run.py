@@ -39,7 +39,7 @@ from ..parts.rope import RotaryEmbedding
 # 8B sizes, 30 tokens 3,685 (4,268), 100 tokens 4,470 (4,815).  In 117 tokens the down projection takes 11.3 us against
 # 13.3, q|k|v with the rotation's launch 14 against 20, whose 12 tiles leave most SMs idle; gate/up would take 27
 # against 21.
-STREAM_MAX = int(os.environ.get("DLGO_PROMPT_STREAM_MAX", 128))
+STREAM_MAX = min(K.GEMM_TC_STREAM_MAX, int(os.environ.get("DLGO_PROMPT_STREAM_MAX", 128)))
 ENABLED = os.environ.get("DLGO_NATIVE_PROMPT", "1") != "0"
 
 
