@@ -11,7 +11,7 @@ sizes, constants, tensors and tile shapes from the parts the model was built
 from, launches what they launch, and steps aside (the parts run one by one) for
 anything else: other blocks, mixers, feed-forwards or norms, float32, head
 sizes the tensor-core attention does not take, per-kernel timing; with
-``DLGO_ORDERED_SUMS`` also for few tokens.
+``DLGO_ORDERED_SUMS`` or without ``DLGO_ATTN_QKV_SUM`` also for few tokens.
 
 ``DLGO_NATIVE_PROMPT=0`` switches it off.
 """
@@ -24,7 +24,7 @@ from typing import Any, Dict, List, Optional
 import torch
 
 from ..csrc import kernels as K
-from ..parts import tensor_core
+from ..parts import attention, tensor_core
 from ..parts.attention import GQAAttention
 from ..parts.block import PreNormBlock
 from ..parts.feedforward import SwiGLU
@@ -78,9 +78,9 @@ class PromptRun:
     def takes(self, ctx: Any, cache: Any) -> bool:
         hd = self.sig[3]
         view = cache.view(self.first)
-        few = ctx.n_tokens <= tensor_core.SKINNY_MAX     # (their K-slices meet in no fixed order)
-        return (not ctx.decode and view is not None and
-                (not few or not (tensor_core.ORDERED_SUMS or ctx.n_tokens > tensor_core.RED_MAX_TOKENS)) and
+        few = ctx.n_tokens <= tensor_core.SKINNY_MAX     # (their K-slices meet in no fixed order, q|k|v's in an fp32 sum)
+        sums = attention._QKV_SUM and not tensor_core.ORDERED_SUMS and ctx.n_tokens <= tensor_core.RED_MAX_TOKENS
+        return (not ctx.decode and view is not None and (sums or not few) and
                 K._profile_events is None and
                 K.attention_prefill_tc_takes(torch.bfloat16, hd, view.page_size) and view.keys.dtype == torch.bfloat16)
 
@@ -138,7 +138,7 @@ class PromptRun:
                 step.splits[j] = 1 if swiglu else splits
             else:
                 step.bn[j], step.pair[j] = lin._tc.many_token_shape(T)
-                if T <= STREAM_MAX and not swiglu and not tensor_core.ORDERED_SUMS and \
+                if T <= STREAM_MAX and not swiglu and (attention._QKV_SUM or j != 0) and not tensor_core.ORDERED_SUMS and \
                         "DLGO_TC_DIRECT_EPILOGUE" not in os.environ:
                     step.form[j] = 2
         if step.form[0] != 0:

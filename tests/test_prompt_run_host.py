@@ -56,3 +56,15 @@ def test_streamed_products_end_where_their_kernel_does(step_of, monkeypatch):
         monkeypatch.delenv("DLGO_PROMPT_STREAM_MAX")
         importlib.reload(prompt_run)
     assert list(step_of(64).form) == [FEW] * 4 and list(step_of(65).form) == [STREAM, STREAM, MANY, STREAM]
+
+
+@pytest.mark.parametrize("tokens", [2, 64, 65, 128, 129])
+def test_the_switch_of_the_projections_fp32_sum_holds_for_prompts(step_of, monkeypatch, tokens):
+    assert bool(step_of(tokens).qkv_sum) == (tokens <= 128)
+    monkeypatch.setattr(attention, "_QKV_SUM", 0)
+    step = step_of(tokens)
+    if tokens <= 64:
+        assert step is None             # part by part
+    else:
+        assert step.form[0] == MANY and not step.qkv_sum and step.fuse_rope == 1
+        assert list(step.form)[1:] == ([STREAM, MANY, STREAM] if tokens <= 128 else [MANY] * 3)
