@@ -38,7 +38,9 @@ from ..parts.rope import RotaryEmbedding
 # whatever the length up to 64); 80 tokens 1,285 and 117 1,323 (tiles of 256 tokens for all products: 1,436 and 1,444); 3.1
 # 8B sizes, 30 tokens 3,685 (4,268), 100 tokens 4,470 (4,815).  In 117 tokens the down projection takes 11.3 us against
 # 13.3, q|k|v with the rotation's launch 14 against 20, whose 12 tiles leave most SMs idle; gate/up would take 27
-# against 21.
+# against 21.  Gate/up of up to 64 tokens is not cut along K, however few tiles a narrow model has: 16 layers of 512, 1,024
+# and 2,048 with inner sizes of 1,024, 2,816 and 4,096 take 546, 587 and 737 us at 30 tokens, and with the K-slices that it gets
+# part by part (where the whole prompt takes 2,160 to 2,190) 621, 633 and 833: its slices meet in a workspace, behind a ticket.
 STREAM_MAX = min(K.GEMM_TC_STREAM_MAX, int(os.environ.get("DLGO_PROMPT_STREAM_MAX", 128)))
 ENABLED = os.environ.get("DLGO_NATIVE_PROMPT", "1") != "0"
 
