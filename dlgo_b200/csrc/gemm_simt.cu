@@ -83,7 +83,7 @@ constexpr int TILE_SMEM = (TILE_RING + BM * BN) * 4;
 
 template <typename T, int EPI, bool VEC>
 __global__ void __launch_bounds__(THREADS, 4)
-gemm_simt_tile_kernel(const T* A, const T* __restrict__ W, void* out, int M, int N, int K, int lda, int ldw, int ldo) {
+gemm_simt_tile_kernel(const T* A, const T* W, void* out, int M, int N, int K, int lda, int ldw, int ldo, int static_w) {
   namespace cg = cooperative_groups;
   constexpr int LROWS = THREADS / 4;
   extern __shared__ __align__(16) float ring[];
@@ -118,6 +118,7 @@ gemm_simt_tile_kernel(const T* A, const T* __restrict__ W, void* out, int M, int
       stage_four<T, VEC>(as + (lrow + LROWS * i) * ROW + lk, A + (size_t)m * lda, k_begin + step * KSTEP + lk, K, m < M);
     }
   };
+  if (!static_w) pdl_wait();    // (W may come from the launch before)
   for (int s = 0; s < STAGES - 1 && s < steps; ++s) load_w(s);
   pdl_wait();
   for (int s = 0; s < STAGES - 1; ++s) {
@@ -234,7 +235,7 @@ template <int MT> struct FewShape {
 
 template <typename T, int EPI, int MT, bool VEC>
 __global__ void __launch_bounds__(FEW_WARPS * 32, 1)
-gemm_simt_few_kernel(const T* A, const T* __restrict__ W, void* out, int M, int N, int K, int lda, int ldw, int ldo) {
+gemm_simt_few_kernel(const T* A, const T* W, void* out, int M, int N, int K, int lda, int ldw, int ldo, int static_w) {
   using S = FewShape<MT>;
   extern __shared__ __align__(16) float ring[];
   pdl_launch_dependents();
@@ -274,6 +275,7 @@ gemm_simt_few_kernel(const T* A, const T* __restrict__ W, void* out, int M, int 
       tile += gridDim.x;
     }
   };
+  if (!static_w) pdl_wait();    // (W may come from the launch before)
   {
     int tile = l_tile, sub = 0;
     for (int i = 0; i < S::STAGES - 1 && i < left; ++i) {
@@ -347,22 +349,22 @@ inline void allow_smem(F* kernel, int bytes) {
 }
 
 template <typename T, int EPI, int MT, bool VEC>
-int launch_few(const T* a, const T* w, void* out, int M, int N, int K, int lda, int ldw, int ldo, cudaStream_t stream) {
+int launch_few(const T* a, const T* w, void* out, int M, int N, int K, int lda, int ldw, int ldo, int static_w, cudaStream_t stream) {
   allow_smem(gemm_simt_few_kernel<T, EPI, MT, VEC>, FewShape<MT>::SMEM);
   const int tiles = (N + FEW_ROWS - 1) / FEW_ROWS, sms = sm_count_of_device();
   launch_kernel(gemm_simt_few_kernel<T, EPI, MT, VEC>, dim3(tiles < sms ? tiles : sms, (M + MT - 1) / MT), dim3(FEW_WARPS * 32),
-                FewShape<MT>::SMEM, stream, a, w, out, M, N, K, lda, ldw, ldo);
+                FewShape<MT>::SMEM, stream, a, w, out, M, N, K, lda, ldw, ldo, static_w);
   return launch_status();
 }
 
 template <typename T, int EPI, bool VEC>
-int launch_tile(const T* a, const T* w, void* out, int M, int N, int K, int lda, int ldw, int ldo, cudaStream_t stream) {
+int launch_tile(const T* a, const T* w, void* out, int M, int N, int K, int lda, int ldw, int ldo, int static_w, cudaStream_t stream) {
   const int quarter = QUARTER * span_length(K), quarters = (K + quarter - 1) / quarter;
   const long long m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
   if (M > 65535 * 64 || m_tiles * n_tiles * quarters > 0x7fffffffLL) return DLGO_ERR_SIZE;
   allow_smem(gemm_simt_tile_kernel<T, EPI, VEC>, TILE_SMEM);
   launch_kernel_cluster(gemm_simt_tile_kernel<T, EPI, VEC>, dim3((unsigned)(m_tiles * n_tiles * quarters)), dim3(THREADS),
-                        TILE_SMEM, stream, dim3(quarters, 1, 1), a, w, out, M, N, K, lda, ldw, ldo);
+                        TILE_SMEM, stream, dim3(quarters, 1, 1), a, w, out, M, N, K, lda, ldw, ldo, static_w);
   return launch_status();
 }
 
@@ -371,30 +373,30 @@ int launch_tile(const T* a, const T* w, void* out, int M, int N, int K, int lda,
 constexpr int FEW_MAX = 16;
 
 template <typename T, int EPI, bool VEC>
-int launch_gemm_simt(const T* a, const T* w, void* out, int M, int N, int K, int lda, int ldw, int ldo, cudaStream_t stream) {
+int launch_gemm_simt(const T* a, const T* w, void* out, int M, int N, int K, int lda, int ldw, int ldo, int static_w, cudaStream_t stream) {
   if (M <= FEW_MAX) {
     if constexpr (VEC) {
-      if (M <= 1) return launch_few<T, EPI, 1, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
-      if (M <= 2) return launch_few<T, EPI, 2, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
-      if (M <= 4) return launch_few<T, EPI, 4, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
+      if (M <= 1) return launch_few<T, EPI, 1, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);
+      if (M <= 2) return launch_few<T, EPI, 2, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);
+      if (M <= 4) return launch_few<T, EPI, 4, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);
     }
-    if (M <= 8) return launch_few<T, EPI, 8, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
-    return launch_few<T, EPI, 16, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
+    if (M <= 8) return launch_few<T, EPI, 8, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);
+    return launch_few<T, EPI, 16, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);
   }
-  return launch_tile<T, EPI, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
+  return launch_tile<T, EPI, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);
 }
 
 template <typename T, bool VEC>
 int by_epilogue(const void* A, const void* W, void* out, int M, int N, int K, int lda, int ldw, int ldo, int epilogue,
-                cudaStream_t stream) {
+                int static_w, cudaStream_t stream) {
   const T* a = (const T*)A;
   const T* w = (const T*)W;
   switch (epilogue) {
     case EPI_STORE:
-      if constexpr (sizeof(T) < 4) return launch_gemm_simt<T, EPI_STORE, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
+      if constexpr (sizeof(T) < 4) return launch_gemm_simt<T, EPI_STORE, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);
       else return DLGO_ERR_SIZE;
-    case EPI_STORE_F32: return launch_gemm_simt<T, EPI_STORE_F32, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
-    case EPI_ADD_F32: return launch_gemm_simt<T, EPI_ADD_F32, VEC>(a, w, out, M, N, K, lda, ldw, ldo, stream);
+    case EPI_STORE_F32: return launch_gemm_simt<T, EPI_STORE_F32, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);
+    case EPI_ADD_F32: return launch_gemm_simt<T, EPI_ADD_F32, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);
     default: return DLGO_ERR_SIZE;
   }
 }
@@ -402,18 +404,19 @@ int by_epilogue(const void* A, const void* W, void* out, int M, int N, int K, in
 }  // namespace dlgo
 
 // A[M, K] (row stride lda), W[N, K] (row stride ldw), both of element type `dtype`;
-// out[M, N] (row stride ldo): epilogue 0 stores `dtype`, 1 stores f32, 2 adds into f32.
+// out[M, N] (row stride ldo): epilogue 0 stores `dtype`, 1 stores f32, 2 adds into f32.  static_w: nothing launched before
+// on the stream writes W (its first pieces are fetched before the launch before has finished).
 DLGO_EXPORT int dlgo_gemm_simt(const void* A, const void* W, void* out, int dtype, int M, int N, int K, int lda,
-                               int ldw, int ldo, int epilogue, cudaStream_t stream) {
+                               int ldw, int ldo, int epilogue, int static_w, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return DLGO_OK;
   if (K <= 0 || lda < K || ldw < K || ldo < N) return DLGO_ERR_SIZE;
   if (dtype == DLGO_F32) {
     // whole aligned pieces of four in every row: asynchronous copies, else element by element
     const bool vec = ((K | lda | ldw) & 3) == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
     if (epilogue == dlgo::EPI_STORE) epilogue = dlgo::EPI_STORE_F32;      // the same
-    return vec ? dlgo::by_epilogue<float, true>(A, W, out, M, N, K, lda, ldw, ldo, epilogue, stream)
-               : dlgo::by_epilogue<float, false>(A, W, out, M, N, K, lda, ldw, ldo, epilogue, stream);
+    return vec ? dlgo::by_epilogue<float, true>(A, W, out, M, N, K, lda, ldw, ldo, epilogue, static_w, stream)
+               : dlgo::by_epilogue<float, false>(A, W, out, M, N, K, lda, ldw, ldo, epilogue, static_w, stream);
   }
-  if (dtype == DLGO_BF16) return dlgo::by_epilogue<__nv_bfloat16, false>(A, W, out, M, N, K, lda, ldw, ldo, epilogue, stream);
+  if (dtype == DLGO_BF16) return dlgo::by_epilogue<__nv_bfloat16, false>(A, W, out, M, N, K, lda, ldw, ldo, epilogue, static_w, stream);
   return DLGO_ERR_DTYPE;
 }

@@ -1397,8 +1397,9 @@ EPI_STORE, EPI_STORE_F32, EPI_ADD_F32 = 0, 1, 2
 
 
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_STORE,
-              out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """x[M, K] . w[N, K]^T on the fp32 pipes; epilogue stores (x's type or fp32) or adds into fp32 ``out``."""
+              out: Optional[torch.Tensor] = None, static_weight: bool = False) -> torch.Tensor:
+    """x[M, K] . w[N, K]^T on the fp32 pipes; epilogue stores (x's type or fp32) or adds into fp32 ``out``.
+    ``static_weight``: no kernel launched before writes ``w``, so that it may be fetched ahead of their end."""
     _need(w, x.dtype, "w")
     if x.dim() != 2 or x.stride(1) != 1:
         raise KernelError("gemm: x must be 2-D with unit inner stride")
@@ -1416,7 +1417,8 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_STORE,
     if out.dtype != want:
         raise KernelError(f"gemm: out must be {want}")
     st = _lib("gemm_simt").dlgo_gemm_simt(_ptr(x), _ptr(w), _ptr(out), _i(dtype_code(x.dtype)), _i(M), _i(N), _i(K),
-                                          _i(x.stride(0)), _i(w.stride(0)), _i(out.stride(0)), _i(epilogue), _stream())
+                                          _i(x.stride(0)), _i(w.stride(0)), _i(out.stride(0)), _i(epilogue),
+                                          _i(1 if static_weight else 0), _stream())
     _check(st, "gemm_simt")
     return out
 
@@ -1936,8 +1938,8 @@ GEMM_TC_STREAM_MAX = 128      # tokens that gemm_tc_stream takes
 
 def gemm_tc_stream(w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, epilogue: int) -> bool:
     """The product of 1 to 128 tokens x[T, K] with a weight w[N, K] by persistent CTAs that stream the weight, in float32
-    [T, N]: ``TC_STORE_F32``, or ``TC_RED_F32`` added into ``out`` (order not fixed).  False where the output's alignment
-    rules it out (nothing ran)."""
+    [T, N]: ``TC_STORE_F32``, or ``TC_RED_F32`` added into ``out`` (order not fixed).  No kernel launched before may write
+    ``w``: it is fetched ahead of their end.  False where the output's alignment rules it out (nothing ran)."""
     for n, t in (("w", w), ("x", x)):
         if not t.is_cuda or t.dtype != torch.bfloat16 or t.dim() != 2 or t.stride(1) != 1:
             raise KernelError(f"gemm_tc_stream: {n} must be a 2-D bfloat16 GPU tensor with unit inner stride")

@@ -1202,3 +1202,20 @@ def test_a_live_position_without_a_page_is_not_written_and_not_read_in_front_of_
     assert torch.equal(got[0], want[0]) and torch.equal(got[2], want[2])
     if not fused:
         assert torch.equal(got[1], attend(stand_in)[0][1])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("M,K_", [(1, 2048), (9, 2048), (40, 2048), (3, 514), (40, 514)])
+def test_gemm_simt_takes_a_weight_that_the_launch_before_makes(dtype, M, K_):
+    """The launch before says at its start that its successor may begin, and is long: its output is another one each time."""
+    k = K()
+    N, dt = 128, DT[dtype]
+    made = torch.zeros(N, K_, device=DEV, dtype=dt)
+    wide = torch.randn(K_, 2048, device=DEV).to(dt)
+    x = torch.randn(M, K_, device=DEV).to(dt)
+    for i in range(20):
+        rows = torch.randn(N, 2048, device=DEV).to(dt) * (0.02 * (i + 1))
+        torch.cuda.synchronize()
+        k.gemm_simt(rows, wide, k.EPI_STORE, made)
+        got = k.gemm_simt(x, made, k.EPI_STORE_F32)
+        assert torch.equal(got, k.gemm_simt(x, made.clone(), k.EPI_STORE_F32))
