@@ -72,22 +72,39 @@ __device__ __forceinline__ void finish(void* out, size_t at, float v) {
 // cluster (as many as are not empty), which evens out the last wave, and meet through distributed shared memory.  A
 // thread's pairs take 128 registers; the sum over a quarter's spans waits in shared memory, a slot per output and thread.
 // Rows lie in a ring of three stages of 16 k, 20 floats apart: the rows that a quarter warp reads are on different banks.
-// Measured on a B200 (TFLOP/s): 567 x 16384 x 2048 41, 567 x 2048 x 8192 35, 64 x 16384 x 2048 34.  Blocks of 128 x 64 with
-// four warps and four stages, two an SM, have as many warps there and more padding: 36, 34 and 19.  64 x 64 outputs of
-// scalar multiply-adds with a synchronous load of every 16 k (before) 4; scalar multiply-adds in this layout 29 where
+// Measured on a B200 (TFLOP/s): 567 x 16384 x 2048 41, 567 x 2048 x 8192 35, 64 x 16384 x 2048 34; 567 x 8192 x 2048 40,
+// 567 x 2048 x 2048 33, 64 x 8192 x 2048 35.  64 x 64 outputs of scalar multiply-adds with a synchronous load of every 16 k
+// (before) gave 24, 11 and 10 for the last three.  Blocks of 128 x 64 with four warps and four stages, two an SM, have as
+// many warps there and more padding: 36, 34 and 19 for the first three; scalar multiply-adds in this layout 29 where
 // packed ones give 38; 8 x 4 outputs per thread with twelve warps an SM and no cluster 36 and 20 for 366 rows.  The order
 // of the multiply-adds and the width of the loads from shared memory change less than 2 %.  The fp32 pipes give 74 at most.
-constexpr int BM = 64, BN = 64, KSTEP = 16, ROW = KSTEP + 4, STAGES = 3, THREADS = 64;
-constexpr int TILE_RING = STAGES * (BM + BN) * ROW;      // floats
-constexpr int TILE_SMEM = (TILE_RING + BM * BN) * 4;
+// (The figures above are VEC's.)  Rows that are no whole aligned pieces of fp32 (odd sizes, and bfloat16, for which this is
+// the stand-in) cannot be copied asynchronously, and a block of two warps waits for the 32 loads a thread that it needs
+// every 16 k: four warps of 8 x 4 outputs a thread instead, which fetch their next 16 values into registers while they
+// multiply; rows 18 floats apart for their pattern.  Measured, us, bfloat16 / fp32 (K 2050 / 2051): 567 x 8192 766 / 716,
+// 200 x 2048 102 / 98, 64 x 1024 48 / 46; two warps of 8 x 8 with loads waited for 1,171 / 1,317 (567 x 8192); one sum per output
+// in 64 x 64 blocks of eight warps (before) 785 / 718, 193 / 186 and 152 / 137.  Eight warps of 4 x 4 outputs: 882 / 874,
+// 124 / 129, 46 / 50; two of 8 x 8 with the loads a step ahead 964 / 772, 120 / 98, 80 / 63; three blocks an SM 870 / 745.
+constexpr int BM = 64, BN = 64, KSTEP = 16;
+template <bool VEC> struct TileShape {
+  static constexpr int THREADS = VEC ? 64 : 128, BLOCKS = 4;                // (blocks an SM)
+  static constexpr int TM = 8, TN = VEC ? 8 : 4;
+  static constexpr int ROW = VEC ? KSTEP + 4 : KSTEP + 2;                   // floats from one staged row to the next
+  static constexpr int STAGES = VEC ? 3 : 2;
+  static constexpr int RING = STAGES * (BM + BN) * ROW;                     // floats
+  static constexpr int SMEM = (RING + BM * BN) * 4;
+  static constexpr int GROUPS = TM * TN / 4;                                // of four outputs of a thread
+  static constexpr int ROWS = THREADS / 16, LOADS = BM / ROWS;              // without VEC: rows at a time, values a thread
+};
 
 template <typename T, int EPI, bool VEC>
-__global__ void __launch_bounds__(THREADS, 4)
+__global__ void __launch_bounds__(TileShape<VEC>::THREADS, TileShape<VEC>::BLOCKS)
 gemm_simt_tile_kernel(const T* A, const T* W, void* out, int M, int N, int K, int lda, int ldw, int ldo, int static_w) {
   namespace cg = cooperative_groups;
-  constexpr int LROWS = THREADS / 4;
+  using S = TileShape<VEC>;
+  constexpr int THREADS = S::THREADS, TM = S::TM, TN = S::TN, ROW = S::ROW, STAGES = S::STAGES, GROUPS = S::GROUPS;
   extern __shared__ __align__(16) float ring[];
-  float4* sums = reinterpret_cast<float4*>(ring + TILE_RING);   // [16][THREADS]: of thread t's output row i, columns 4 h .. 4 h + 3 at 2 i + h
+  float4* sums = reinterpret_cast<float4*>(ring + S::RING);   // [GROUPS][THREADS]: of thread t's output row i, columns 4 h .. 4 h + 3 at i * TN / 4 + h
   pdl_launch_dependents();
   cg::cluster_group cl = cg::this_cluster();
   const int quarters = (int)cl.num_blocks(), quarter = (int)cl.block_rank();
@@ -95,60 +112,84 @@ gemm_simt_tile_kernel(const T* A, const T* W, void* out, int M, int N, int K, in
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m_tiles = (M + BM - 1) / BM;                      // blocks of the same weight rows follow one another
   const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
-  const int tm = lane >> 2;                                   // rows tm + 8 i
-  const int tn = warp * 32 + (lane & 3) * 2;                  // columns tn + (j & 1) + 8 (j >> 1)
-  const int lrow = tid >> 2, lk = (tid & 3) * 4;              // loading
+  // a thread's outputs: rows tm + 8 i, columns tn + col_of(j)
+  const int tm = VEC ? lane >> 2 : tid >> 4, tn = VEC ? warp * 32 + (lane & 3) * 2 : tid & 15;
+  auto col_of = [](int j) { return VEC ? (j & 1) + 8 * (j >> 1) : 16 * j; };
   const int span = span_length(K);
   const int k_begin = quarter * QUARTER * span, k_end = min(K, k_begin + QUARTER * span);
   const int steps = (k_end - k_begin + KSTEP - 1) / KSTEP;    // (quarters that exist are not empty)
   const int span_steps = span / KSTEP;
-  auto load_w = [&](int step) {
-    float* ws = ring + ((step % STAGES) * (BM + BN) + BM) * ROW;
+  // VEC: four k of rows vrow + 16 i straight into the ring
+  const int vrow = tid >> 2, vk = (tid & 3) * 4;
+  auto copy_rows = [&](const T* rows, int ld, int first, int count, int step, int at) {
 #pragma unroll
-    for (int i = 0; i < BN / LROWS; ++i) {
-      const int n = n0 + lrow + LROWS * i;
-      stage_four<T, VEC>(ws + (lrow + LROWS * i) * ROW + lk, W + (size_t)n * ldw, k_begin + step * KSTEP + lk, K, n < N);
+    for (int i = 0; i < 4; ++i) {
+      const int r = vrow + 16 * i;
+      stage_four<T, true>(ring + ((step % STAGES) * (BM + BN) + at + r) * ROW + vk, rows + (size_t)(first + r) * ld,
+                          k_begin + step * KSTEP + vk, K, first + r < count);
     }
   };
-  auto load_a = [&](int step) {
-    float* as = ring + (step % STAGES) * (BM + BN) * ROW;
+  // else: one k of rows erow + S::ROWS i, through registers
+  const int erow = tid >> 4, ek = tid & 15;
+  T next[2][VEC ? 1 : S::LOADS];                              // (A, W)
+  auto fetch_rows = [&](const T* rows, int ld, int first, int count, int step, T (&x)[VEC ? 1 : S::LOADS]) {
+    const int k = k_begin + step * KSTEP + ek;
 #pragma unroll
-    for (int i = 0; i < BM / LROWS; ++i) {
-      const int m = m0 + lrow + LROWS * i;
-      stage_four<T, VEC>(as + (lrow + LROWS * i) * ROW + lk, A + (size_t)m * lda, k_begin + step * KSTEP + lk, K, m < M);
+    for (int i = 0; i < S::LOADS; ++i) {
+      const int r = first + erow + S::ROWS * i;
+      x[i] = r < count && k < K ? rows[(size_t)r * ld + k] : from_float<T>(0.f);
     }
+  };
+  auto put_rows = [&](int step) {
+#pragma unroll
+    for (int o = 0; o < 2; ++o)
+#pragma unroll
+      for (int i = 0; i < S::LOADS; ++i)
+        ring[((step % STAGES) * (BM + BN) + o * BM + erow + S::ROWS * i) * ROW + ek] = to_float(next[o][i]);
   };
   if (!static_w) pdl_wait();    // (W may come from the launch before)
-  for (int s = 0; s < STAGES - 1 && s < steps; ++s) load_w(s);
-  pdl_wait();
-  for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < steps) load_a(s);
-    copies_commit();
+  if constexpr (VEC) {
+    for (int s = 0; s < STAGES - 1 && s < steps; ++s) copy_rows(W, ldw, n0, N, s, BM);
+    pdl_wait();
+    for (int s = 0; s < STAGES - 1; ++s) {
+      if (s < steps) copy_rows(A, lda, m0, M, s, 0);
+      copies_commit();
+    }
+  } else {
+    fetch_rows(W, ldw, n0, N, 0, next[1]);
+    pdl_wait();
+    fetch_rows(A, lda, m0, M, 0, next[0]);
+    put_rows(0);
   }
-  unsigned long long acc[8][8];
+  unsigned long long acc[TM][TN];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
   int in_span = 0;
   bool first = true;
   for (int s = 0; s < steps; ++s) {
-    copies_wait<STAGES - 2>();
+    if constexpr (VEC) copies_wait<STAGES - 2>();
     __syncthreads();            // stage s is in place, and every warp is past stage s - 1
-    if (s + STAGES - 1 < steps) {
-      load_w(s + STAGES - 1);
-      load_a(s + STAGES - 1);
+    if constexpr (VEC) {
+      if (s + STAGES - 1 < steps) {
+        copy_rows(W, ldw, n0, N, s + STAGES - 1, BM);
+        copy_rows(A, lda, m0, M, s + STAGES - 1, 0);
+      }
+      copies_commit();
+    } else if (s + 1 < steps) {
+      fetch_rows(W, ldw, n0, N, s + 1, next[1]);
+      fetch_rows(A, lda, m0, M, s + 1, next[0]);
     }
-    copies_commit();
     const float* as = ring + ((s % STAGES) * (BM + BN) + tm) * ROW;
     const float* ws = ring + ((s % STAGES) * (BM + BN) + BM + tn) * ROW;
     // two neighbours of k at a time; the next two are on their way from shared memory while these are multiplied
-    unsigned long long a[2][8], b[2][8];
-    auto fetch = [&](int k, unsigned long long (&x)[8], unsigned long long (&y)[8]) {
+    unsigned long long a[2][TM], b[2][TN];
+    auto fetch = [&](int k, unsigned long long (&x)[TM], unsigned long long (&y)[TN]) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) y[j] = *reinterpret_cast<const unsigned long long*>(ws + ((j & 1) + 8 * (j >> 1)) * ROW + k);
+      for (int j = 0; j < TN; ++j) y[j] = *reinterpret_cast<const unsigned long long*>(ws + col_of(j) * ROW + k);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const unsigned long long*>(as + 8 * i * ROW + k);
+      for (int i = 0; i < TM; ++i) x[i] = *reinterpret_cast<const unsigned long long*>(as + 8 * i * ROW + k);
     };
     fetch(0, a[0], b[0]);
 #pragma unroll
@@ -156,18 +197,21 @@ gemm_simt_tile_kernel(const T* A, const T* W, void* out, int M, int N, int K, in
       const int now = (k >> 1) & 1;
       if (k + 2 < KSTEP) fetch(k + 2, a[now ^ 1], b[now ^ 1]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          const int j = (i & 1) ? 7 - jj : jj;          // (a row after another shares an operand at the turn)
+        for (int jj = 0; jj < TN; ++jj) {
+          const int j = (i & 1) ? TN - 1 - jj : jj;     // (a row after another shares an operand at the turn)
           fma_two(acc[i][j], a[now][i], b[now][j]);
         }
     }
+    if constexpr (!VEC) {
+      if (s + 1 < steps) put_rows(s + 1);               // (where stage s - 1 was)
+    }
     if (++in_span == span_steps || s == steps - 1) {
 #pragma unroll
-      for (int g = 0; g < 16; ++g) {
+      for (int g = 0; g < GROUPS; ++g) {
         float4 v = first ? make_float4(0.f, 0.f, 0.f, 0.f) : sums[g * THREADS + tid];
-        unsigned long long* q = &acc[g >> 1][(g & 1) * 4];
+        unsigned long long* q = &acc[g / (TN / 4)][g % (TN / 4) * 4];
         v.x += pair_sum(q[0]); v.y += pair_sum(q[1]); v.z += pair_sum(q[2]); v.w += pair_sum(q[3]);
         sums[g * THREADS + tid] = v;
         q[0] = q[1] = q[2] = q[3] = 0ull;
@@ -177,42 +221,49 @@ gemm_simt_tile_kernel(const T* A, const T* W, void* out, int M, int N, int K, in
     }
   }
   // Every block of the cluster finishes a share of the tile; what is added into is fetched while the others arrive.
-  float old[4][4];
+  auto store = [&](int g, const float4& v, const float* added) {            // group g of this thread's outputs
+    const float f[4] = {v.x, v.y, v.z, v.w};
+    const int m = m0 + tm + 8 * (g / (TN / 4)), n = n0 + tn + col_of(g % (TN / 4) * 4);
+    if (m >= M) return;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int ne = n + col_of(e);
+      if (ne >= N) continue;
+      if (added != nullptr) ((float*)out)[(size_t)m * ldo + ne] = added[e] + f[e];
+      else finish<T, EPI>(out, (size_t)m * ldo + ne, f[e]);
+    }
+  };
+  if (quarters == 1) {
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) store(g, sums[g * THREADS + tid], nullptr);
+    return;
+  }
+  float old[GROUPS / 4][4];
   if (EPI == EPI_ADD_F32 && quarters == 4) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int g = quarter + 4 * i, m = m0 + tm + 8 * (g >> 1), n = n0 + tn + 16 * (g & 1);
+    for (int i = 0; i < GROUPS / 4; ++i) {
+      const int g = quarter + 4 * i, m = m0 + tm + 8 * (g / (TN / 4)), n = n0 + tn + col_of(g % (TN / 4) * 4);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int ne = n + (e & 1) + 8 * (e >> 1);
-        old[i][e] = m < M && ne < N ? ((const float*)out)[(size_t)m * ldo + ne] : 0.f;
-      }
+      for (int e = 0; e < 4; ++e)
+        old[i][e] = m < M && n + col_of(e) < N ? ((const float*)out)[(size_t)m * ldo + n + col_of(e)] : 0.f;
     }
   }
-  if (quarters > 1) cl.sync();
+  cl.sync();
   auto share = [&](int g, const float* added) {
     float4 v = *cl.map_shared_rank(sums + g * THREADS + tid, 0);
     for (int q = 1; q < quarters; ++q) {
       const float4 u = *cl.map_shared_rank(sums + g * THREADS + tid, q);
       v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
     }
-    const float f[4] = {v.x, v.y, v.z, v.w};
-    const int m = m0 + tm + 8 * (g >> 1), n = n0 + tn + 16 * (g & 1);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int ne = n + (e & 1) + 8 * (e >> 1);
-      if (m >= M || ne >= N) continue;
-      if (added != nullptr) ((float*)out)[(size_t)m * ldo + ne] = added[e] + f[e];
-      else finish<T, EPI>(out, (size_t)m * ldo + ne, f[e]);
-    }
+    store(g, v, added);
   };
   if (quarters == 4) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) share(quarter + 4 * i, EPI == EPI_ADD_F32 ? old[i] : nullptr);
+    for (int i = 0; i < GROUPS / 4; ++i) share(quarter + 4 * i, EPI == EPI_ADD_F32 ? old[i] : nullptr);
   } else {
-    for (int g = quarter; g < 16; g += quarters) share(g, nullptr);
+    for (int g = quarter; g < GROUPS; g += quarters) share(g, nullptr);
   }
-  if (quarters > 1) cl.sync();  // nobody leaves while its sums may still be read
+  cl.sync();                    // nobody leaves while its sums may still be read
 }
 
 // ------------------------------------------------------------------- few rows
@@ -359,12 +410,13 @@ int launch_few(const T* a, const T* w, void* out, int M, int N, int K, int lda, 
 
 template <typename T, int EPI, bool VEC>
 int launch_tile(const T* a, const T* w, void* out, int M, int N, int K, int lda, int ldw, int ldo, int static_w, cudaStream_t stream) {
+  using S = TileShape<VEC>;
   const int quarter = QUARTER * span_length(K), quarters = (K + quarter - 1) / quarter;
   const long long m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
   if (M > 65535 * 64 || m_tiles * n_tiles * quarters > 0x7fffffffLL) return DLGO_ERR_SIZE;
-  allow_smem(gemm_simt_tile_kernel<T, EPI, VEC>, TILE_SMEM);
-  launch_kernel_cluster(gemm_simt_tile_kernel<T, EPI, VEC>, dim3((unsigned)(m_tiles * n_tiles * quarters)), dim3(THREADS),
-                        TILE_SMEM, stream, dim3(quarters, 1, 1), a, w, out, M, N, K, lda, ldw, ldo, static_w);
+  allow_smem(gemm_simt_tile_kernel<T, EPI, VEC>, S::SMEM);
+  launch_kernel_cluster(gemm_simt_tile_kernel<T, EPI, VEC>, dim3((unsigned)(m_tiles * n_tiles * quarters)), dim3(S::THREADS), S::SMEM,
+                        stream, dim3(quarters, 1, 1), a, w, out, M, N, K, lda, ldw, ldo, static_w);
   return launch_status();
 }
 
@@ -372,9 +424,16 @@ int launch_tile(const T* a, const T* w, void* out, int M, int N, int K, int lda,
 // it takes for 17 to 64 rows alike.
 constexpr int FEW_MAX = 16;
 
+// Up to 64 k have two spans: one warp of a few-row block works.  Where it can also not copy asynchronously and has more than
+// two tiles to take in turn, the tile kernel is the better one: 1 / 16 rows of 8192 x 37 6.7 / 10.1 us, tiles 5.3; of
+// 2048 x 37, less than a tile a block, 2.7 / 4.2 and 3.9.
+inline bool few_rows(bool vec, int M, int N, int K) {
+  return M <= FEW_MAX && (vec || K > 64 || N <= 2 * FEW_ROWS * sm_count_of_device());
+}
+
 template <typename T, int EPI, bool VEC>
 int launch_gemm_simt(const T* a, const T* w, void* out, int M, int N, int K, int lda, int ldw, int ldo, int static_w, cudaStream_t stream) {
-  if (M <= FEW_MAX) {
+  if (few_rows(VEC, M, N, K)) {
     if constexpr (VEC) {
       if (M <= 1) return launch_few<T, EPI, 1, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);
       if (M <= 2) return launch_few<T, EPI, 2, VEC>(a, w, out, M, N, K, lda, ldw, ldo, static_w, stream);

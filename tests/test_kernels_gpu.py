@@ -1219,3 +1219,23 @@ def test_gemm_simt_takes_a_weight_that_the_launch_before_makes(dtype, M, K_):
         k.gemm_simt(rows, wide, k.EPI_STORE, made)
         got = k.gemm_simt(x, made, k.EPI_STORE_F32)
         assert torch.equal(got, k.gemm_simt(x, made.clone(), k.EPI_STORE_F32))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("N,K_", [(145, 37), (64, 514), (130, 2051), (4800, 37), (4800, 64), (4800, 65)])
+def test_gemm_simt_of_rows_that_are_no_aligned_pieces(dtype, N, K_):
+    """Element by element: few rows and tiles add in the same order (with few k and many outputs, tiles take few rows too).
+    The bound is that of the aligned rows above."""
+    k = K()
+    torch.manual_seed(N + K_)
+    x = torch.randn(193, K_, device=DEV).to(DT[dtype])
+    w = torch.randn(N, K_ + 1, device=DEV).to(DT[dtype])[:, :K_].contiguous()
+    ref = x.double() @ w.double().t()
+    bound = (x.double().abs() @ w.double().abs().t()) * (K_ / 32 + 32) * 2.0 ** -24
+    got = k.gemm_simt(x, w, k.EPI_STORE_F32)
+    assert ((got.double() - ref).abs() <= bound).all()
+    for n in (1, 8, 9, 16, 17, 64, 65, 129):
+        acc = torch.randn(n, N + 3, device=DEV)
+        before = acc.clone()
+        k.gemm_simt(x[:n].contiguous(), w, k.EPI_ADD_F32, acc[:, :N])
+        assert torch.equal(acc[:, :N], before[:, :N] + got[:n]) and torch.equal(acc[:, N:], before[:, N:])
