@@ -16,6 +16,8 @@
 // fp32 residual in place (models/llm/forward.go:163,169).
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "async_copy.cuh"
 #include "common.cuh"
 
@@ -389,19 +391,36 @@ gemm_simt_few_kernel(const T* A, const T* W, void* out, int M, int N, int K, int
   copies_wait<0>();
 }
 
+// What a launch asks the runtime once per device (of the first 64; others are asked each time): together half a
+// microsecond of host time.
+constexpr int DEVICES = 64;
+inline int current_device() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : DEVICES;
+}
 inline int sm_count_of_device() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  static std::atomic<int> counts[DEVICES];
+  const int dev = current_device();
+  int n = dev < DEVICES ? counts[dev].load(std::memory_order_relaxed) : 0;
+  if (n > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  if (dev < DEVICES) counts[dev].store(n, std::memory_order_relaxed);
   return n;
 }
+// `allowed`: a bit per device, of this kernel
 template <typename F>
-inline void allow_smem(F* kernel, int bytes) {
-  cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+inline void allow_smem(std::atomic<unsigned long long>& allowed, F* kernel, int bytes) {
+  const int dev = current_device();
+  const unsigned long long bit = dev < DEVICES ? 1ull << dev : 0;
+  if (allowed.load(std::memory_order_acquire) & bit) return;
+  if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+    allowed.fetch_or(bit, std::memory_order_release);
 }
 
 template <typename T, int EPI, int MT, bool VEC>
 int launch_few(const T* a, const T* w, void* out, int M, int N, int K, int lda, int ldw, int ldo, int static_w, cudaStream_t stream) {
-  allow_smem(gemm_simt_few_kernel<T, EPI, MT, VEC>, FewShape<MT>::SMEM);
+  static std::atomic<unsigned long long> allowed{0};
+  allow_smem(allowed, gemm_simt_few_kernel<T, EPI, MT, VEC>, FewShape<MT>::SMEM);
   const int tiles = (N + FEW_ROWS - 1) / FEW_ROWS, sms = sm_count_of_device();
   launch_kernel(gemm_simt_few_kernel<T, EPI, MT, VEC>, dim3(tiles < sms ? tiles : sms, (M + MT - 1) / MT), dim3(FEW_WARPS * 32),
                 FewShape<MT>::SMEM, stream, a, w, out, M, N, K, lda, ldw, ldo, static_w);
@@ -414,7 +433,8 @@ int launch_tile(const T* a, const T* w, void* out, int M, int N, int K, int lda,
   const int quarter = QUARTER * span_length(K), quarters = (K + quarter - 1) / quarter;
   const long long m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
   if (M > 65535 * 64 || m_tiles * n_tiles * quarters > 0x7fffffffLL) return DLGO_ERR_SIZE;
-  allow_smem(gemm_simt_tile_kernel<T, EPI, VEC>, S::SMEM);
+  static std::atomic<unsigned long long> allowed{0};
+  allow_smem(allowed, gemm_simt_tile_kernel<T, EPI, VEC>, S::SMEM);
   launch_kernel_cluster(gemm_simt_tile_kernel<T, EPI, VEC>, dim3((unsigned)(m_tiles * n_tiles * quarters)), dim3(S::THREADS), S::SMEM,
                         stream, dim3(quarters, 1, 1), a, w, out, M, N, K, lda, ldw, ldo, static_w);
   return launch_status();
