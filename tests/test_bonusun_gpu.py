@@ -255,6 +255,41 @@ def test_sinks_in_every_attention_kernel(H, G, hd, window, act_dtype):
             assert worst(o, want) < tol, (split, worst(o, want))
 
 
+@pytest.mark.parametrize("window", [0, 1, 33, 100, 1000, -64, -96, -700])
+@pytest.mark.parametrize("H, G, hd", [(4, 2, 64), (6, 1, 128), (12, 1, 64), (20, 1, 128)])
+def test_sinks_and_split_weights_in_even_shares(H, G, hd, window):
+    """Sequences in parts of several blocks, alone in one, several to a block, all with sinks; a sliding window and chunks,
+    both beginning inside a tile or at its edge; more than eight heads to a key head."""
+    from dlgo_b200.csrc import kernels as K
+    g = torch.Generator().manual_seed(H * hd + abs(window))
+    PS, lens, scale = 64, [4000, 1, 2, 64, 65, 129, 400, 33, 1, 1, 2500], hd ** -0.5
+    T, N = len(lens), 23
+    kp, vp = (torch.randn(N, G, PS, hd, generator=g).to(torch.bfloat16) for _ in range(2))
+    table = torch.full((T, -(-max(lens) // PS)), -1, dtype=torch.int32)
+    first = [n - 1 - (n - 1) % -window if window < 0 else (max(0, n - window) if window else 0) for n in lens]
+    for i, n in enumerate(lens):        # (pages before the first visible key are gone)
+        for p in range(first[i] // PS, -(-n // PS)):
+            table[i, p] = int(torch.randint(0, N, (1,), generator=g))
+    sink = torch.linspace(-30.0, 9.0, H)
+    q = (2 * torch.randn(T, H * hd, generator=g)).to(torch.bfloat16)
+    want = torch.zeros(T, H * hd, dtype=torch.float64)
+    for i, n in enumerate(lens):
+        lo = first[i] // PS * PS
+        rows = [torch.cat([x[int(table[i, p])].transpose(0, 1) for p in range(lo // PS, -(-n // PS))])[first[i] - lo:n - lo]
+                for x in (kp, vp)]
+        want[i] = attention_reference(q[i].view(H, hd), rows, scale, 0, sink, H, G).reshape(-1)
+    scratch = torch.full((K.attention_decode_shares_scratch(H, G, hd),), float("nan"), device=DEV)
+    tickets = torch.zeros(T * G * ((H // G + 7) // 8), dtype=torch.int32, device=DEV)
+    for split, tol in ((False, 2e-2), (True, 6e-3)):        # (as in the kernels above: two bfloat16 terms of a weight, one)
+        for _ in range(2):
+            o = K.attention_decode_mma(q.to(DEV), H * hd, T, kp.to(DEV), vp.to(DEV), table.to(DEV), i32(range(T)),
+                                       i32([n - 1 for n in lens]),
+                                       torch.full((T, H * hd), float("nan"), dtype=torch.bfloat16, device=DEV), H, G, hd, scale, window,
+                                       0, 32, scratch, sink=sink.to(DEV), split=split, tickets=tickets)
+            assert torch.isfinite(o).all() and worst(o, want) < tol, (split, worst(o, want))
+            assert not tickets.any()
+
+
 @pytest.mark.parametrize("T", [3, 200])
 def test_router_with_groups_scored_by_two(T):
     """Groups whose largest score is not their largest sum, choice scores that are negative, weights without correction."""

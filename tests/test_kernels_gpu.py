@@ -1239,3 +1239,31 @@ def test_gemm_simt_of_rows_that_are_no_aligned_pieces(dtype, N, K_):
         before = acc.clone()
         k.gemm_simt(x[:n].contiguous(), w, k.EPI_ADD_F32, acc[:, :N])
         assert torch.equal(acc[:, :N], before[:, :N] + got[:n]) and torch.equal(acc[:, N:], before[:, N:])
+
+
+def test_decode_attention_in_even_shares_of_the_most_sequences_and_tiles():
+    """2,048 sequences of up to 131,072 keys, 592 blocks: a block's place times the tiles needs more than 32 bits.  All pages
+    come from 64, so a sequence's result is known from how often it holds each.  Error: a weight's and the output's
+    rounding, 2^-9 each of a weighted mean of |v|."""
+    k = K()
+    torch.manual_seed(0)
+    B, hd, PS, n_pages, per = k.SHARES_MAX_SEQUENCES, 64, 64, 64, 2048
+    kp, vp = (torch.randn(n_pages, 1, PS, hd, device=DEV).to(torch.bfloat16) for _ in range(2))
+    q = (2 * torch.randn(B, hd, device=DEV)).to(torch.bfloat16)
+    table = torch.randint(0, n_pages, (B, per), device=DEV, dtype=torch.int32)
+    held = per - torch.arange(B, device=DEV) % 5                     # pages of each sequence
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert int(held.sum()) * (PS // 32) >= (2 ** 32 - 1) // (4 * sms)
+    tickets = torch.zeros(B, dtype=torch.int32, device=DEV)
+    scratch = torch.full((k.attention_decode_shares_scratch(1, 1, hd),), float("nan"), device=DEV)
+    out = torch.full((B, hd), float("nan"), device=DEV, dtype=torch.bfloat16)
+    k.attention_decode_mma(q, hd, B, kp, vp, table, torch.arange(B, dtype=torch.int32, device=DEV), (held * PS - 1).int(), out, 1, 1,
+                           hd, hd ** -0.5, 0, 0, 32, scratch, tickets=tickets)
+    assert not tickets.any()
+    live = torch.arange(per, device=DEV)[None] < held[:, None]
+    times = torch.zeros(B, n_pages, device=DEV, dtype=torch.float64).scatter_add_(1, table.long(), live.double())
+    s = (q.double() @ kp.view(-1, hd).double().t() * hd ** -0.5).view(B, n_pages, PS)
+    w = torch.exp(s - s.amax((1, 2), keepdim=True)) * times[:, :, None]
+    w = (w / w.sum((1, 2), keepdim=True)).view(B, -1)
+    v = vp.view(-1, hd).double()
+    assert ((out.double() - w @ v).abs() <= 2.0 ** -8 * (w @ v.abs()) + 1e-4).all()
