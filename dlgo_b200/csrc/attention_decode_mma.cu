@@ -418,12 +418,15 @@ attention_decode_shares_kernel(DecMmaParams p, int B, int* tickets) {
   }
   __syncthreads();
   const unsigned P = first[B];
-  // A block per sequence where the longest does not outlast the whole launch by more than sharing costs: a tile of one
+  // A block per sequence where none is longer than a block's least run; and, where there are too few blocks for two a
+  // sequence, where the longest does not outlast the whole launch by more than sharing costs: a tile of one
   // block takes some 0.5 us while all stream, the launch streams 6.5 MB/us, and parts, tickets and sums take 5 us.
   // (Measured on a B200, a block per sequence / shares, us: 32 sequences of 2,048, heads of 128, 53 / 55; of 256 to
-  // 4,096 87 / 61; 16 of 64 to 2,048 42 / 20; 64 of 128 to 1,024, heads of 64, 21 / 23; of 128 to 4,096 68 / 55.)
-  const bool whole_only = B <= (int)gridDim.x &&
-      (float)longest * 0.5f <= (float)P * ((float)gridDim.y * TK * HD * 4 / 6.5e6f) + 5.f;
+  // 4,096 87 / 61; 16 of 64 to 2,048 42 / 20; 64 of 128 to 1,024, heads of 64, 21 / 23; of 128 to 4,096 68 / 55.  Where two
+  // blocks a sequence fit, one takes, us a layer in a step at the 3B sizes, 4 to 5 more for 13 to 16 sequences of 500 keys
+  // and 5 more for 18 of 1,000.)
+  const bool whole_only = B <= (int)gridDim.x && (longest <= DS_MIN_TILES ||
+      (2 * B > (int)gridDim.x && (float)longest * 0.5f <= (float)P * ((float)gridDim.y * TK * HD * 4 / 6.5e6f) + 5.f));
   const unsigned nb = whole_only ? B : min(gridDim.x, max(1u, (P + DS_MIN_TILES - 1) / DS_MIN_TILES));   // (<= P: no run is empty)
   if (blockIdx.x >= nb) return;
   const bool narrow = P < 0xffffffffu / nb;           // (a division of 64 bits takes a microsecond's tenth)
@@ -446,6 +449,19 @@ attention_decode_shares_kernel(DecMmaParams p, int B, int* tickets) {
     const int pg0 = (max(lo, first[s]) + rebase) * TK / p.page_size, pg1 = (min(hi, first[s + 1]) - 1 + rebase) * TK / p.page_size;
     for (int pg = pg0 + tid * 32; pg < pg1 + 32; pg += DM_THREADS * 32)
       asm volatile("prefetch.global.L1 [%0];" ::"l"(row + min(pg, pg1)));
+    // A hint that pulls a short run's keys and values into L2, up to three rounds a warp.  (Heads of 64, two to eight
+    // sequences of 300 to 9,000 keys, us a layer: 0.3 to 1.1 less; longer runs 0.1 to 0.3 more; heads of 128 0.5 to 1 more.)
+    if (HD <= 64 && hi - lo <= 3 * DM_WARPS) {
+      const int at = max(lo, first[s]), upto = min(hi, first[s + 1]);
+      for (int tile = at + ((warp - (at - lo)) & (DM_WARPS - 1)); tile < upto; tile += DM_WARPS) {
+        const int key = (tile + rebase) * TK, page = readable_page(row, key / p.page_size);
+        const size_t base = (((size_t)page * p.Hkv + kvh) * p.page_size + key % p.page_size) * HD;
+        for (int ln = lane; ln < TK * HD * 2 / 128; ln += 32) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)(p.kpages + base) + (size_t)ln * 128));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)(p.vpages + base) + (size_t)ln * 128));
+        }
+      }
+    }
     constexpr int LN = (RH * 4 + 127) / 128;
     if (p.parts != nullptr && tid >= 64 && tid < 64 + 2 * LN) {
       const float* tbl = (tid - 64 < LN ? p.cos_t : p.sin_t) + (size_t)pos * RH;
@@ -603,12 +619,14 @@ attention_decode_shares_kernel(DecMmaParams p, int B, int* tickets) {
         if (first[seq] < lo || first[seq + 1] > hi) {
           const int n = block_of(first[seq + 1] - 1) - block_of(first[seq]) + 1;
           int* ticket = tickets + (size_t)seq * gridDim.y + blockIdx.y;
-          __threadfence();            // the block's parts, behind the barrier, before the ticket
-          if (atomicAdd(ticket, 1) == n - 1) {
+          // releases the block's parts, which are behind the barrier; acquires, for the whole block behind the next one,
+          // those of the blocks before it (two full fences around a relaxed add: 0.4 us a layer more)
+          int before;
+          asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(before) : "l"(ticket) : "memory");
+          if (before == n - 1) {
             *ticket = 0;              // for the next launch
             mine = 1;
           }
-          __threadfence();
         }
         last[tid] = mine;
       }

@@ -1267,3 +1267,15 @@ def test_decode_attention_in_even_shares_of_the_most_sequences_and_tiles():
     w = (w / w.sum((1, 2), keepdim=True)).view(B, -1)
     v = vp.view(-1, hd).double()
     assert ((out.double() - w @ v).abs() <= 2.0 ** -8 * (w @ v.abs()) + 1e-4).all()
+
+
+@pytest.mark.parametrize("hq,hkv,hd", [(8, 2, 64), (6, 2, 128)])
+@pytest.mark.parametrize("case", ["least run", "a key more", "one of many", "two blocks each", "no two blocks each", "short runs", "longer runs"])
+def test_decode_attention_in_even_shares_at_the_edges_of_its_rules(hq, hkv, hd, case):
+    """Whole sequences to a block or shares of them, runs with a hint and without."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    fit = (4 if hd <= 64 else 2) * sms // hkv // 2          # sequences for which two blocks each are resident
+    lens = {"least run": [256] * 9, "a key more": [257] * 9, "one of many": [1] * 17 + [288], "two blocks each": [300] * fit,
+            "no two blocks each": [300] * (fit + 1), "short runs": [32 * 12 * 2 * fit // 3] * 3, "longer runs": [32 * 13 * 2 * fit // 3] * 3}[case]
+    out, ref = _attention_case("bfloat16", hq, hkv, hd, [(n - 1, 1) for n in lens], n_splits=0, decode=True, kernel="shares")
+    torch.testing.assert_close(out, ref, atol=2e-2, rtol=2e-2)
