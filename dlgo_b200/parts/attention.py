@@ -109,23 +109,37 @@ class GQAAttention(Mixer):
         return -self.chunk if self.chunk else 0
 
     # -------------------------------------------------------------------- forward
-    def _decode_slices(self, ctx: Any, cache: Any, T: int, group: int, pages: int):
-        """(page slices per sequence, scratch, counters) of the decode kernels: slices so that every SM has
-        several blocks (whole waves: rounded down); 2..8 slices form a thread-block cluster and combine
-        through distributed shared memory, more (one very long sequence alone) go through scratch memory."""
+    def _decode_slices(self, T: int, pages: int, sms: int) -> tuple:
+        """(page slices per sequence of the decode kernels, how many would fit): slices so that every SM has several
+        blocks (whole waves: rounded down), no more than pages; 2..8 form a thread-block cluster and combine through
+        distributed shared memory, more (few very long sequences) go through scratch memory."""
         # (as many blocks as are resident at once: four per SM, two for heads above 64, whose kernel takes twice
         # the registers; measured on a B200 at the layer sizes of Llama 3.2 3B, heads of 128, batch 8: 4 slices
         # in one wave 1.83 ms a step, 8 slices in two waves 2.04 ms)
-        blocks = _DECODE_BLOCKS or (4 if self.head_dim <= 64 else 2) * _sm_count(cache.keys.device)
-        base_blocks = T * self.num_kv_heads * ((group + 3) // 4)
-        n_splits = max(1, min(pages, blocks // base_blocks))
-        scratch = counters = None
+        blocks = _DECODE_BLOCKS or (4 if self.head_dim <= 64 else 2) * sms
+        group = self.num_heads // self.num_kv_heads
+        fit = max(1, blocks // (T * self.num_kv_heads * ((group + 3) // 4)))
+        n_splits = max(1, min(pages, fit))
         if n_splits > _CLUSTER_MAX and pages <= 64 and _CLUSTER_MAX > 1:
             n_splits = _CLUSTER_MAX
-        if n_splits > _CLUSTER_MAX:
-            scratch = ctx.scratch("attention", K.attention_scratch_floats(T, self.num_heads, self.head_dim, n_splits))
-            counters = ctx.zeros("attention_counters", T * self.num_kv_heads * ((group + 3) // 4))
-        return n_splits, scratch, counters
+        return n_splits, fit
+
+    def _even_shares(self, T: int, n_splits: int, fit: int) -> bool:
+        """Whether the blocks of a head share the keys of all of the step's sequences evenly instead."""
+        # Where so few slices fit that the longest sequence decides how long the launch takes, or more than a cluster
+        # holds.  Measured on a B200 in whole steps at the layer sizes of Llama 3.2 1B (heads of 64) and 3B (128), 8 kv
+        # heads, us a layer, shares less slices, for sequences of one length / of mixed ones:
+        #   heads of 128, 1 fits (20 to 32 sequences of 100 to 3,900):   -31 to -1    / 64 to 2,000 -27 to -21
+        #                 2 fit (13 to 18):                              -17 to +1.1  / -15 to -10
+        #                 3 fit (10 and 11; clusters of 3 pack badly from 12 on, -40 to -4):   -5 to +2.7 / -9 to -8
+        #                 4 fit (8 sequences): 100 keys +1.7, 1,000 +2.3, 3,900 -2.7 / 323 to 3,900 -12: slices
+        #   more than 8 slices, heads of 64: one sequence of 4,150 to 100,000 -11 to -9; two -6 to -4 / 300 and 9,000 -4;
+        #                 three to eight of 4,150 to 15,000 -4 to +1.8 / one of 9,000 beside 300 each -10 to -2
+        #   more than 8 slices, heads of 128: one -6 to -4; two -2.5 to +2.5 / -4; three and four -4 to +0.9 / -19 to -14
+        # Heads of 64 have twice the blocks: one slice (64 of up to 1,024 keys: 1.200 ms a step / 1.211 with shares) and two (32:
+        # 13 us / 16) are the better ones there.
+        return bool(_SHARES and _MMA_KEYS == 32 and T <= K.SHARES_MAX_SEQUENCES and
+                    (n_splits > 8 or (n_splits <= 3 and self.head_dim > 64)))
 
     def fuses_prompt_rope(self, ctx: Any, cache: Any, positions: Mapping[str, PositionEncoding]) -> bool:
         """Whether this step's q|k|v projection rotates and appends in its own epilogue: a prompt step in
@@ -146,20 +160,18 @@ class GQAAttention(Mixer):
         longest = ctx.capacity if ctx.captured else ctx.max_len
         pages = max(1, (longest + cache.page_size - 1) // cache.page_size)
         decode_kernel = ctx.decode and K.attention_decode_takes(act, self.head_dim, cache.page_size)
-        n_splits, scratch, counters = self._decode_slices(ctx, cache, T, group, pages) if decode_kernel else (1, None, None)
+        n_splits, fit = self._decode_slices(T, pages, _sm_count(cache.keys.device)) if decode_kernel else (1, 1)
         mma = (decode_kernel and _MMA_KEYS > 0 and
                K.attention_decode_mma_takes(act, self.head_dim, cache.page_size, n_splits))
-        # Even shares of all sequences' keys (n_splits 0) where a sequence would get few slices, so that the longest
-        # decides how long the launch takes, or more than a cluster holds.  Measured on a B200 in a whole step, ms, slices
-        # / shares: 8B sizes, 32 sequences (1 slice) 6.23 / 5.16; 3B, 16 (2) 2.45 / 2.11; 1B, two long ones (37) 1.06 /
-        # 0.98.  Four slices are better at heads of 128 (8B, 8 sequences of up to 1,024 keys: 12 us a layer / 15), and
-        # at heads of 64, whose blocks are twice as many, one (1B, 64 of up to 1,024 keys: 1.200 ms / 1.211) and two (32: 13
-        # us / 16).
-        if (mma and _SHARES and _MMA_KEYS == 32 and T <= K.SHARES_MAX_SEQUENCES and
-                (n_splits > 8 or (n_splits <= 3 and self.head_dim > 64))):
+        scratch = counters = None
+        if mma and self._even_shares(T, n_splits, fit):
             n_splits = 0
             scratch = ctx.scratch("attention", K.attention_decode_shares_scratch(self.num_heads, self.num_kv_heads, self.head_dim))
             counters = ctx.zeros("attention_tickets", T * self.num_kv_heads * ((group + 7) // 8))
+        elif n_splits > _CLUSTER_MAX:       # (on the tensor cores only with DLGO_ATTN_SHARES=0 or 16 keys an iteration)
+            scratch = ctx.scratch("attention", K.attention_scratch_floats(T, self.num_heads, self.head_dim, n_splits))
+            if not mma:
+                counters = ctx.zeros("attention_counters", T * self.num_kv_heads * ((group + 3) // 4))
         return decode_kernel, mma, n_splits, scratch, counters, pages
 
     def _attend(self, qkv: torch.Tensor, ctx: Any, cache: Any, out: torch.Tensor, decode_kernel: bool, mma: bool,

@@ -344,8 +344,8 @@ def test_ordered_sums_make_bfloat16_decoding_repeatable_bit_for_bit(batch8, monk
 def test_default_cache_sizing_and_a_very_long_capacity(batch8):
     # no max_tokens: the cache is sized from the context (131072 positions here).  Captured steps are sized for
     # the reach they are asked for: these short sequences replay the graph for 4,096 positions; the same step
-    # through the graph for the whole context (2048 pages a sequence: decode attention takes its many-slices
-    # path through scratch memory) gives the same logits
+    # through the graph for the whole context (2048 pages a sequence: decode attention takes even shares of all
+    # keys instead of slices) gives the same logits
     from dlgo_b200.engine import graphs
     from dlgo_b200.engine.engine import Engine
     d, reqs, refs = batch8
