@@ -39,3 +39,11 @@ def test_slices_allocate_as_they_did(plan):
     assert plan(32, 8, 64, 4, 4096) == (8, {})
     assert plan(32, 8, 64, 64, 4096) == (1, {})
     assert plan(32, 8, 64, 2, 16384, torch.float32) == (37, {"attention": K.attention_scratch_floats(2, 32, 64, 37), "attention_counters": 16})
+
+
+@pytest.mark.parametrize("T", [1, 4, 8])
+@pytest.mark.parametrize("reach", [40, 64, 128, 190])
+def test_few_pages_do_not_make_even_shares(plan, T, reach):
+    """Heads of 128: shares where few slices FIT, not where a short sequence has no more pages."""
+    assert plan(24, 8, 128, T, reach) == (min(-(-reach // 64), 296 // (8 * T)), {})
+    assert plan(24, 8, 128, 10, 4096)[0] == 0 and plan(24, 8, 128, 37, 4096)[0] == 0 and plan(24, 8, 128, 9, 4096)[0] == 4
