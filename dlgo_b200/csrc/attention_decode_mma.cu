@@ -360,10 +360,12 @@ __global__ void __launch_bounds__(DM_THREADS, HD <= 64 ? 4 : 2) attention_decode
 // that takes a sequence's last ticket adds them up; nobody waits for another block.  Every block works out the cut
 // from the positions (the step's own inputs) while its predecessor drains.
 // Measured on a B200: 32 sequences of 256 to 4,096 keys, 8 kv heads of 128 (301 MB) 61 us, 49 of them streaming at 6.1
-// TB/s; one slice per sequence 87 us, a cluster of two 85.  In a step at the 8B sizes 6.23 -> 5.16 ms, 3B sizes with 16
-// sequences of 64 to 2,048 keys 2.45 -> 2.11, 1B sizes with two of 14,000 to 17,800 1.06 -> 0.98 (37 slices combined by
-// a second kernel before).  Clusters stay where they leave a block two or three rounds: their sums meet faster (16
-// sequences of 128 to 1,024 keys, heads of 64: 9 us against 14).
+// TB/s; one slice per sequence 87 us, a cluster of two 85.  In a step at the 8B sizes 6.22 -> 5.17 ms, 3B sizes with 16
+// sequences of 64 to 2,048 keys 2.50 -> 2.12, 1B sizes with two of 14,000 to 17,800 1.05 -> 0.97 (37 slices combined by
+// a second kernel before).  Where heads of 64 would get up to eight slices, clusters that leave a block two or three rounds
+// stay: their sums meet faster (16 sequences of 128 to 1,024 keys: 9 us against 14).  Stamps of six sequences of 4,150 keys
+// of heads of 64, us: 1.5 of the cut are not hidden, queries 1.5, tiles 7, merge 1, ticket 1, sum of 13 parts 4 to 6; eight
+// parts in flight instead of four shorten that sum by 1 where there are 20 and more and cost 0.5 where there are few.
 // Up to DS_SEGS sequences at a time go through one round: queries (rotated here where the projection's sum comes in,
 // new keys and values appended) to shared memory, the warps' tiles of all of them without a barrier, one merge.
 constexpr int DS_SEGS = 4;

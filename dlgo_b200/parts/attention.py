@@ -139,7 +139,7 @@ class GQAAttention(Mixer):
         # Heads of 64 have twice the blocks: one slice (64 of up to 1,024 keys: 1.200 ms a step / 1.211 with shares) and two (32:
         # 13 us / 16) are the better ones there.
         return bool(_SHARES and _MMA_KEYS == 32 and T <= K.SHARES_MAX_SEQUENCES and
-                    (n_splits > 8 or (n_splits <= 3 and self.head_dim > 64)))
+                    (n_splits > 8 or (fit <= 3 and self.head_dim > 64)))
 
     def fuses_prompt_rope(self, ctx: Any, cache: Any, positions: Mapping[str, PositionEncoding]) -> bool:
         """Whether this step's q|k|v projection rotates and appends in its own epilogue: a prompt step in
