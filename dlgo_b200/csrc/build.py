@@ -36,6 +36,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "attention_decode": ["attention_decode.cu"],
     "attention_decode_mma": ["attention_decode_mma.cu"],
     "hoststep": ["hoststep.cu"],
+    "packrows": ["packrows.cu"],
     "attention_prefill_tc": ["attention_prefill_tc.cu"],
     "decode_layers": ["decode_layers.cu"],
     "prompt_layers": ["prompt_layers.cu"],

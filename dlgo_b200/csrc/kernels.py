@@ -2356,6 +2356,25 @@ def filter_draw(logits: torch.Tensor, temperature: float, top_k: int, top_p: flo
 
 
 # ------------------------------------------------------------------ host side of a decode step
+_pack_rows = None
+
+
+def pack_rows(parts: list, rows: list, width: int) -> Optional[torch.Tensor]:
+    """A list of lists of whole numbers one after another, then the last ``width`` numbers of each of ``rows`` (-1 behind
+    a shorter one), as one int32 tensor on the host; ``None`` where that is not what they are (csrc/packrows.cu).
+    Measured for 64 rows of 64 numbers: 29 us; flattened in Python and packed by ``struct`` 72."""
+    global _pack_rows
+    if _pack_rows is None:
+        # (the interpreter's lock stays held: the numbers are read out of Python objects)
+        fn = ctypes.PyDLL(build.ensure_built(["packrows"])["packrows"]).dlgo_pack_rows
+        fn.argtypes = [ctypes.py_object, ctypes.py_object, _i, _p, _ll]
+        fn.restype = _i
+        _pack_rows = fn
+    room = sum(map(len, parts)) + width * len(rows)
+    out = torch.empty((room,), dtype=torch.int32)
+    return out if _pack_rows(parts, rows, width, out.data_ptr(), room) == 1 else None
+
+
 class HostStep:
     """The runtime calls of a decode step's launch as one native call: inputs out of a pinned buffer,
     an event that frees the buffer, the captured graph."""

@@ -82,8 +82,13 @@ def draw_on_device(logits: torch.Tensor, cfg: SamplerConfig, requests: torch.Ten
 
 def _int32_rows(parts: Sequence[Sequence[int]], rows: Sequence[Sequence[int]], width: int, device: torch.device) -> torch.Tensor:
     """``parts`` one after another, then the last ``width`` numbers of each of ``rows`` (-1 behind a shorter one), as
-    one int32 tensor on the device: one copy.  (64 rows of 64 tokens: 70 us of host time and one copy, against 310 us
-    for a tensor of nested lists.)"""
+    one int32 tensor on the device: one copy.  Lists of whole numbers are read natively; whatever else a list can be made
+    of is flattened here.  (64 rows of 64 tokens: 29 us of host time natively, 72 us here, 310 us for a tensor of nested
+    lists.)"""
+    if all(type(p) is list for p in parts):
+        host = K.pack_rows(list(parts), list(rows), width)
+        if host is not None:
+            return host.to(device, non_blocking=True) if host.numel() else torch.empty((0,), dtype=torch.int32, device=device)
     flat: list = []
     for p in parts:
         flat.extend(p)          # (+= would add an array's numbers to the list's)

@@ -48,3 +48,15 @@ def test_the_sampler_takes_iterators_and_deques_and_refuses_no_rows(monkeypatch)
         DeviceSampler().sample(logits, cfg, [8, 9], [1, 2], [])
     with pytest.raises(ValueError):
         DeviceSampler().sample(logits, cfg, [8, 9], [1], rows)
+
+
+def test_numbers_that_are_read_natively():
+    """Lists of whole numbers of 32 bits are, edges and all; anything else is left to the general way, untouched."""
+    from dlgo_b200.csrc import kernels as K
+    low, high = -2 ** 31, 2 ** 31 - 1
+    assert K.pack_rows([[1, True], [low]], [[], [high], list(range(7))], 3).tolist() == [1, 1, low, -1, -1, -1, high, -1, -1, 4, 5, 6]
+    assert K.pack_rows([[np.int64(5)]], [], 3).tolist() == [5] and K.pack_rows([[]], [], 3).tolist() == []
+    for odd in ([[1.0]], [[high + 1]], [[low - 1]], [["1"]], [[None]], [(1, 2)]):
+        assert K.pack_rows(odd, [], 3) is None and K.pack_rows([[1]], odd, 3) is None
+    row = iter([1, 2])
+    assert K.pack_rows([[1]], [row], 3) is None and list(row) == [1, 2]
