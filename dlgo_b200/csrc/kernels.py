@@ -1398,7 +1398,8 @@ EPI_STORE, EPI_STORE_F32, EPI_ADD_F32 = 0, 1, 2
 
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_STORE,
               out: Optional[torch.Tensor] = None, static_weight: bool = False) -> torch.Tensor:
-    """x[M, K] . w[N, K]^T on the fp32 pipes; epilogue stores (x's type or fp32) or adds into fp32 ``out``.
+    """x[M, K] . w[N, K]^T on the fp32 pipes, or, for more than 16 rows of fp32, by pieces on the tensor cores
+    (csrc/gemm_split.cuh); epilogue stores (x's type or fp32) or adds into fp32 ``out``.
     ``static_weight``: no kernel launched before writes ``w``, so that it may be fetched ahead of their end."""
     _need(w, x.dtype, "w")
     if x.dim() != 2 or x.stride(1) != 1:
