@@ -493,23 +493,50 @@ inline bool split_takes(const void* W, int M, int N, int K, int ldw) {
 }
 inline int split_tile_rows(int M) { return M <= 64 ? 64 : 128; }
 
+// Clusters of `blocks` blocks of the kernel that are resident at once; asked for once per device and size.  (A cluster stays
+// within a group of SMs, so that larger ones leave some idle.)
+template <int BN, bool ADD>
+int resident_clusters(int blocks) {
+  static std::atomic<int> counts[DEVICES][SPLIT_SPANS + 1];
+  const int sms = sm_count_of_device(), dev = current_device();
+  if (blocks <= 1) return sms;
+  int n = dev < DEVICES ? counts[dev][blocks].load(std::memory_order_relaxed) : 0;
+  if (n > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks * sms);
+  cfg.blockDim = dim3(SPLIT_THREADS);
+  cfg.dynamicSmemBytes = SplitShape<BN>::SMEM;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_split_kernel<BN, ADD>, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    return sms / blocks > 1 ? sms / blocks : 1;
+  }
+  if (dev < DEVICES) counts[dev][blocks].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 template <int BN, bool ADD>
 int launch_split_tile(const float* a, const float* w, float* out, int M, int N, int K, int lda, int ldw, int ldo, int a_aligned,
                       int static_w, uint8_t* scratch, cudaStream_t stream) {
   using S = SplitShape<BN>;
-  const int span = split_span_length(K), spans = (K + span - 1) / span, chunks = (K + SPLIT_K - 1) / SPLIT_K, sms = sm_count_of_device();
+  const int span = split_span_length(K), spans = (K + span - 1) / span, chunks = (K + SPLIT_K - 1) / SPLIT_K;
   const long long m_tiles = (M + BN - 1) / BN, tiles = m_tiles * ((N + 127) / 128);
   if (m_tiles > 65535 || tiles * spans > 0x7fffffffLL) return DLGO_ERR_SIZE;
+  static std::atomic<unsigned long long> allowed{0};
+  allow_smem(allowed, gemm_split_kernel<BN, ADD>, S::SMEM);
   int block_spans = SPLIT_SPANS;
   long long best = -1;
-  for (int per : {8, 2, 1}) {
-    const long long blocks = (spans + per - 1) / per, rounds = (tiles * blocks + sms - 1) / sms;
-    const long long cost = rounds * ((chunks + blocks - 1) / blocks + 4);
+  for (int per : {8, 2, 1}) {           // rounds of blocks times what one takes, its start and end as long as four times 64 k
+    const int blocks = (spans + per - 1) / per, at_once = resident_clusters<BN, ADD>(blocks);
+    const long long cost = (tiles + at_once - 1) / at_once * ((chunks + blocks - 1) / blocks + 4);
     if (best < 0 || cost < best) { best = cost; block_spans = per; }
   }
   const int blocks = (spans + block_spans - 1) / block_spans;
-  static std::atomic<unsigned long long> allowed{0};
-  allow_smem(allowed, gemm_split_kernel<BN, ADD>, S::SMEM);
   launch_kernel(split_rows_kernel<BN>, dim3(chunks, (unsigned)m_tiles), dim3(256), 0, stream, a, scratch, M, K, lda, a_aligned);
   launch_kernel_cluster(gemm_split_kernel<BN, ADD>, dim3((unsigned)(tiles * blocks)), dim3(SPLIT_THREADS), S::SMEM, stream,
                         dim3(blocks, 1, 1), a, (const uint8_t*)scratch, w, out, M, N, K, lda, ldw, ldo, block_spans, static_w);
