@@ -77,16 +77,13 @@ __device__ __forceinline__ void add_two(float& a, float& b, float x, float y) {
       : "f"(x), "f"(y));
 }
 
-// the sum on the fp32 pipes, for outputs whose pieces are no numbers
-__device__ __noinline__ float split_plain_sum(const float* a, const float* w, int K) {
-  float even = 0.f, odd = 0.f;
-  int k = 0;
-  for (; k + 1 < K; k += 2) {
-    even = fmaf(a[k], w[k], even);
-    odd = fmaf(a[k + 1], w[k + 1], odd);
-  }
-  if (k < K) even = fmaf(a[k], w[k], even);
-  return even + odd;
+// the sum on the fp32 pipes, for outputs whose pieces are no numbers (inlined: a call costs the kernel registers, and 366 x
+// 16384 x 2048 8 %)
+__device__ __forceinline__ float split_plain_sum(const float* a, const float* w, int K) {
+  float sum = 0.f;
+#pragma unroll 1
+  for (int k = 0; k < K; ++k) sum = fmaf(a[k], w[k], sum);
+  return sum;
 }
 
 template <bool ADD>
@@ -128,15 +125,19 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* A, uint8_t
 // them, whose blocks are then a cluster and meet through distributed shared memory, each finishing a part of the tile.
 //   warps 0-7   read the sums of a chunk out of tensor memory (a warp's own 32 lanes, half of the columns) into registers
 //   warps 8-15  fetch the weight, two blocks of 64 k ahead, split it and lay the pieces out with the 128-byte swizzle
-//   warp 16     one thread issues the MMAs: per 16 k high by high, high by middle | low (one instruction, twice as wide),
-//               middle by high | middle, low by high; sums that take part in the same instruction lie side by side
+//   warp 16     one thread issues the MMAs of high pieces
+//   warp 18     one thread issues the others: per 16 k high by middle | low (one instruction, twice as wide), middle by
+//               high | middle, low by high; sums that take part in the same instruction lie side by side.  (One thread for
+//               all waited for the chunk's sums to be read before it issued what does not need that: 200 -> 182 us)
 //   warp 17     one thread copies the tiles of x
 // Tensor memory: the sums of high products, the two others, and a place for the spans before.
-// Bound by the chain weight -> pieces -> MMAs in two stages of shared memory (the tensor pipe is 30 to 40 % busy), by
-// shared memory itself, and by rounds of blocks where there are few.  Measured on a B200, us a product in a row of them with
-// x's split (on the fp32 pipes): 17 x 16384 x 2048 47 (121), 64 x 3072 x 2048 21 (53), 64 x 2048 x 8192 55 (177), 128 x 16384
-// x 2048 77 (226), 366 x 16384 x 2048 199 (613), 366 x 2048 x 8192 162 (340), 1500 x 2048 x 8192 441 (1,196: 114 TFLOP/s
-// against 42, where the fp32 pipes give 74 at most).
+// Bound by the chain weight -> pieces -> MMAs in two stages of shared memory, in which pieces are written and read at the
+// same time (without the writes 10 % less; the tensor pipe is 40 % busy).  Measured on a B200, us a product in a row of them
+// with x's split (on the fp32 pipes): 17 x 16384 x 2048 47 (121), 64 x 3072 x 2048 22 (53), 64 x 2048 x 8192 54 (177), 128 x
+// 16384 x 2048 61 (226), 366 x 3072 x 2048 57 (142), 366 x 16384 x 2048 170 (613), 366 x 2048 x 8192 125 (340), 1500 x 2048 x
+// 8192 362 (1,196: 139 TFLOP/s against 42, where the fp32 pipes give 74 at most).  Stages of 32 k (four, rows of 64 bytes)
+// took 23 % longer for 128 rows a tile and 48 % for 64; 64 rows a tile for all sizes 30 % longer; the weight hinted into L2
+// ahead, or fetched past L1, changed nothing or lost.
 template <int BN> struct SplitShape {
   static constexpr int STAGES = BN >= 128 ? 2 : 3;
   static constexpr int W_PIECE = 128 * 128, X_PIECE = BN * 128;               // bytes: rows of 64 bfloat16
@@ -145,7 +146,7 @@ template <int BN> struct SplitShape {
   static constexpr int TMEM = BN >= 128 ? 512 : 256;                           // 4 x BN columns
   static_assert(4 * BN <= TMEM && 2 * BN * 128 * 4 <= STAGES * STAGE, "");
 };
-constexpr int SPLIT_THREADS = 18 * 32;
+constexpr int SPLIT_THREADS = 19 * 32;
 
 // contiguous bytes into shared memory, counted on `bar` (16-byte aligned, a multiple of 16 bytes)
 __device__ __forceinline__ void split_bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -187,7 +188,7 @@ gemm_split_kernel(const float* A, const uint8_t* x_tiles, const float* W, float*
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 9);
-      mbar_init(&empty[s], 1);
+      mbar_init(&empty[s], 2);
     }
     mbar_init(high_full, 1);
     mbar_init(high_empty, 8);
@@ -268,46 +269,49 @@ gemm_split_kernel(const float* A, const uint8_t* x_tiles, const float* W, float*
       }
     }
   } else if (warp == 16) {
-    if (elect_one()) {
-      constexpr uint32_t one = umma_idesc_bf16(128, BN), two = umma_idesc_bf16(128, 2 * BN);
+    if (elect_one()) {                                        // the products of high pieces
+      constexpr uint32_t one = umma_idesc_bf16(128, BN);
+      const uint64_t dw0 = umma_desc_k_sw128(smem_u32(smem)), dx0 = umma_desc_k_sw128(smem_u32(smem + 3 * S::W_PIECE));
       bool ok = true;
-      int in_span = 0, sp = 0;
-      for (int c = 0; c < chunks && ok; ++c) {
-        const int s = c % STAGES;
-        if (!mbar_wait(&full[s], (c / STAGES) & 1, abort_flag)) break;
-        tc_fence_after_sync();
-        const uint32_t base = smem_u32(smem + s * S::STAGE);
-        uint64_t dw[3], dx[2];
-#pragma unroll
-        for (int p = 0; p < 3; ++p) dw[p] = umma_desc_k_sw128(base + p * S::W_PIECE);
-#pragma unroll
-        for (int p = 0; p < 2; ++p) dx[p] = umma_desc_k_sw128(base + 3 * S::W_PIECE + p * S::X_PIECE);
+      for (int c = 0, s = 0, turn = 0; c < chunks && ok; ++c) {
+        if (!mbar_wait(&full[s], turn, abort_flag)) break;
+        const uint64_t at = (uint64_t)(s * (S::STAGE >> 4));
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           if (c + half > 0 && !mbar_wait(high_empty, half ^ 1, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
 #pragma unroll
-          for (int kk = 0; kk < 2; ++kk) umma_bf16(tmem, dw[0] + 2 * (2 * half + kk), dx[0] + 2 * (2 * half + kk), one, kk != 0);
+          for (int k = 0; k < 2; ++k) umma_bf16(tmem, dw0 + at + 2 * (2 * half + k), dx0 + at + 2 * (2 * half + k), one, k != 0);
           umma_commit(high_full);
-          if (half == 0 && in_span == 0 && c > 0) {
-            if (!mbar_wait(rest_empty, (sp - 1) & 1, abort_flag)) { ok = false; break; }
-            tc_fence_after_sync();
-          }
-#pragma unroll
-          for (int kk = 0; kk < 2; ++kk) {
-            const uint64_t k = 2 * (2 * half + kk);
-            umma_bf16(t_rest, dw[0] + k, dx[1] + k, two, (half | kk | in_span) != 0);
-            umma_bf16(t_rest, dw[1] + k, dx[0] + k, two, true);
-            umma_bf16(t_rest + BN, dw[2] + k, dx[0] + k, one, true);
-          }
         }
-        if (!ok) break;
+        umma_commit(&empty[s]);
+        if (++s == STAGES) { s = 0; turn ^= 1; }
+      }
+    }
+  } else if (warp == 18) {
+    if (elect_one()) {                                        // the others
+      constexpr uint32_t one = umma_idesc_bf16(128, BN), two = umma_idesc_bf16(128, 2 * BN);
+      const uint64_t dw0 = umma_desc_k_sw128(smem_u32(smem)), dx0 = umma_desc_k_sw128(smem_u32(smem + 3 * S::W_PIECE));
+      constexpr uint64_t WP = S::W_PIECE >> 4, XP = S::X_PIECE >> 4;
+      int in_span = 0, sp = 0;
+      for (int c = 0, s = 0, turn = 0; c < chunks; ++c) {
+        if (!mbar_wait(&full[s], turn, abort_flag)) break;
+        if (in_span == 0 && c > 0 && !mbar_wait(rest_empty, (sp - 1) & 1, abort_flag)) break;
+        tc_fence_after_sync();
+        const uint64_t dw = dw0 + (uint64_t)(s * (S::STAGE >> 4)), dx = dx0 + (uint64_t)(s * (S::STAGE >> 4));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          umma_bf16(t_rest, dw + 2 * k, dx + XP + 2 * k, two, (k | in_span) != 0);
+          umma_bf16(t_rest, dw + WP + 2 * k, dx + 2 * k, two, true);
+          umma_bf16(t_rest + BN, dw + 2 * WP + 2 * k, dx + 2 * k, one, true);
+        }
         umma_commit(&empty[s]);
         if (in_span == span_chunks - 1 || c == chunks - 1) umma_commit(rest_full);
         if (++in_span == span_chunks) {
           in_span = 0;
           ++sp;
         }
+        if (++s == STAGES) { s = 0; turn ^= 1; }
       }
     }
   } else {
