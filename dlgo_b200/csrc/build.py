@@ -59,7 +59,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "rglru_tc": ["rglru_tc.cu"],
 }
 _HEADERS = ["common.cuh", "attention_noalloc.h", "attention_combine.cuh", "attention_decode_tiles.cuh", "tcgen05.cuh",
-            "async_copy.cuh", "gemm_split.cuh", "ssd.cuh", "ssd_state.cuh"]
+            "async_copy.cuh", "ssd.cuh", "ssd_state.cuh"]
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 BASE_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-shared", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]

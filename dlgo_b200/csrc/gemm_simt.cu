@@ -1,12 +1,12 @@
-// y[M, N] = x[M, K] . W[N, K]^T of 32-bit values, for every size.
+// y[M, N] = x[M, K] . W[N, K]^T on the fp32 pipes (FFMA), for every size.
 //
-// This is the contraction of the true 32-bit path, the plain counterpart the bfloat16
-// tensor-core kernel is checked against, and the stand-in where that kernel refuses a
-// size.  It runs on the fp32 pipes (FFMA) here, or, for many rows of 32 bits, as sums of
-// exact products of pieces on the tensor cores (gemm_split.cuh), never in a reduced-precision mode.
-// The reference contracts one weight row with the activation vector per output (blas/blas.go:152-196, models/llm/forward.go:224,286,296-298).
+// This is the contraction of the true 32-bit path (no tensor cores, no
+// reduced-precision matrix mode), the plain counterpart the tensor-core kernel
+// is checked against, and the stand-in where the tensor-core kernel refuses a
+// size.  The reference contracts one weight row with the activation vector per
+// output (blas/blas.go:152-196, models/llm/forward.go:224,286,296-298).
 //
-// The order of an output's sum on the fp32 pipes is fixed by K alone and the same in both kernels below, so a row's result does not
+// The order of an output's sum is fixed by K alone and the same in both kernels below, so a row's result does not
 // depend on the other rows of the launch, nor on which kernel ran.  K is cut into 16 spans of equal length (a multiple of
 // 32; the last ones may be short or empty).  Within a span the products of even k and those of odd k are two running
 // sums: one packed fp32 pair, since fma.rn.f32x2 takes two neighbours of k straight from rows as they lie, so nothing is
@@ -20,7 +20,6 @@
 
 #include "async_copy.cuh"
 #include "common.cuh"
-#include "gemm_split.cuh"
 
 namespace dlgo {
 
@@ -481,101 +480,16 @@ int by_epilogue(const void* A, const void* W, void* out, int M, int N, int K, in
   }
 }
 
-// Which products are summed by pieces on the tensor cores (gemm_split.cuh): more than FEW_MAX rows of 32 bits (few rows are
-// bound by reading the weight, and splitting it costs a block of them more than the multiply-adds that it saves: 1 row of
-// 16384 x 2048 21.6 us here, 26.7 by pieces through mma.sync, 2048 x 2048 3.7 and 5.6), weights whose rows are aligned pieces
-// of four, of SPLIT_MIN values and more.  DLGO_F32_SPLIT=0 switches it off: then a row's bits do not depend on whether the
-// step it came in had more than FEW_MAX rows.
-constexpr long long SPLIT_MIN = 1ll << 20;
-inline bool split_takes(const void* W, int M, int N, int K, int ldw) {
-  static const bool on = [] { const char* e = getenv("DLGO_F32_SPLIT"); return e == nullptr || e[0] != '0'; }();
-  return on && M > FEW_MAX && ((K | ldw) & 3) == 0 && ((uintptr_t)W & 15) == 0 && (long long)N * K >= SPLIT_MIN;
-}
-inline int split_tile_rows(int M) { return M <= 64 ? 64 : 128; }
-
-// Clusters of `blocks` blocks of the kernel that are resident at once; asked for once per device and size.  (A cluster stays
-// within a group of SMs, so that larger ones leave some idle.)
-template <int BN, bool ADD>
-int resident_clusters(int blocks) {
-  static std::atomic<int> counts[DEVICES][SPLIT_SPANS + 1];
-  const int sms = sm_count_of_device(), dev = current_device();
-  if (blocks <= 1) return sms;
-  int n = dev < DEVICES ? counts[dev][blocks].load(std::memory_order_relaxed) : 0;
-  if (n > 0) return n;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks * sms);
-  cfg.blockDim = dim3(SPLIT_THREADS);
-  cfg.dynamicSmemBytes = SplitShape<BN>::SMEM;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = blocks;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm_split_kernel<BN, ADD>, &cfg) != cudaSuccess || n < 1) {
-    cudaGetLastError();
-    return sms / blocks > 1 ? sms / blocks : 1;
-  }
-  if (dev < DEVICES) counts[dev][blocks].store(n, std::memory_order_relaxed);
-  return n;
-}
-
-template <int BN, bool ADD>
-int launch_split_tile(const float* a, const float* w, float* out, int M, int N, int K, int lda, int ldw, int ldo, int a_aligned,
-                      int static_w, uint8_t* scratch, cudaStream_t stream) {
-  using S = SplitShape<BN>;
-  const int span = split_span_length(K), spans = (K + span - 1) / span, chunks = (K + SPLIT_K - 1) / SPLIT_K;
-  const long long m_tiles = (M + BN - 1) / BN, tiles = m_tiles * ((N + 127) / 128);
-  if (m_tiles > 65535 || tiles * spans > 0x7fffffffLL) return DLGO_ERR_SIZE;
-  static std::atomic<unsigned long long> allowed{0};
-  allow_smem(allowed, gemm_split_kernel<BN, ADD>, S::SMEM);
-  int block_spans = SPLIT_SPANS;
-  long long best = -1;
-  for (int per : {8, 2, 1}) {           // rounds of blocks times what one takes, its start and end as long as four times 64 k
-    const int blocks = (spans + per - 1) / per, at_once = resident_clusters<BN, ADD>(blocks);
-    const long long cost = (tiles + at_once - 1) / at_once * ((chunks + blocks - 1) / blocks + 4);
-    if (best < 0 || cost < best) { best = cost; block_spans = per; }
-  }
-  const int blocks = (spans + block_spans - 1) / block_spans;
-  launch_kernel(split_rows_kernel<BN>, dim3(chunks, (unsigned)m_tiles), dim3(256), 0, stream, a, scratch, M, K, lda, a_aligned);
-  launch_kernel_cluster(gemm_split_kernel<BN, ADD>, dim3((unsigned)(tiles * blocks)), dim3(SPLIT_THREADS), S::SMEM, stream,
-                        dim3(blocks, 1, 1), a, (const uint8_t*)scratch, w, out, M, N, K, lda, ldw, ldo, block_spans, static_w);
-  return launch_status();
-}
-
-template <bool ADD>
-int launch_split(const float* a, const float* w, float* out, int M, int N, int K, int lda, int ldw, int ldo, int static_w, uint8_t* scratch,
-                 cudaStream_t stream) {
-  const int al = (lda & 3) == 0 && ((uintptr_t)a & 15) == 0;
-  if (scratch == nullptr || ((uintptr_t)scratch & 15) != 0) return DLGO_ERR_ALIGN;
-  if (split_tile_rows(M) == 64) return launch_split_tile<64, ADD>(a, w, out, M, N, K, lda, ldw, ldo, al, static_w, scratch, stream);
-  return launch_split_tile<128, ADD>(a, w, out, M, N, K, lda, ldw, ldo, al, static_w, scratch, stream);
-}
-
 }  // namespace dlgo
-
-// Bytes of scratch (16-byte aligned) that dlgo_gemm_simt wants for these arguments: the pieces of A's rows; 0: none
-DLGO_EXPORT long long dlgo_gemm_simt_scratch(const void* W, int dtype, int M, int N, int K, int ldw) {
-  if (dtype != DLGO_F32 || M <= 0 || N <= 0 || K <= 0 || !dlgo::split_takes(W, M, N, K, ldw)) return 0;
-  const int bn = dlgo::split_tile_rows(M);
-  return (long long)((M + bn - 1) / bn) * ((K + dlgo::SPLIT_K - 1) / dlgo::SPLIT_K) * (3 * bn * 128);
-}
 
 // A[M, K] (row stride lda), W[N, K] (row stride ldw), both of element type `dtype`;
 // out[M, N] (row stride ldo): epilogue 0 stores `dtype`, 1 stores f32, 2 adds into f32.  static_w: nothing launched before
 // on the stream writes W (its first pieces are fetched before the launch before has finished).
 DLGO_EXPORT int dlgo_gemm_simt(const void* A, const void* W, void* out, int dtype, int M, int N, int K, int lda,
-                               int ldw, int ldo, int epilogue, int static_w, void* scratch, cudaStream_t stream) {
+                               int ldw, int ldo, int epilogue, int static_w, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return DLGO_OK;
   if (K <= 0 || lda < K || ldw < K || ldo < N) return DLGO_ERR_SIZE;
   if (dtype == DLGO_F32) {
-    if (epilogue < 0 || epilogue > dlgo::EPI_ADD_F32) return DLGO_ERR_SIZE;
-    if (dlgo::split_takes(W, M, N, K, ldw)) {
-      const float *a = (const float*)A, *w = (const float*)W;
-      return epilogue == dlgo::EPI_ADD_F32
-                 ? dlgo::launch_split<true>(a, w, (float*)out, M, N, K, lda, ldw, ldo, static_w, (uint8_t*)scratch, stream)
-                 : dlgo::launch_split<false>(a, w, (float*)out, M, N, K, lda, ldw, ldo, static_w, (uint8_t*)scratch, stream);
-    }
     // whole aligned pieces of four in every row: asynchronous copies, else element by element
     const bool vec = ((K | lda | ldw) & 3) == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
     if (epilogue == dlgo::EPI_STORE) epilogue = dlgo::EPI_STORE_F32;      // the same
@@ -584,12 +498,4 @@ DLGO_EXPORT int dlgo_gemm_simt(const void* A, const void* W, void* out, int dtyp
   }
   if (dtype == DLGO_BF16) return dlgo::by_epilogue<__nv_bfloat16, false>(A, W, out, M, N, K, lda, ldw, ldo, epilogue, static_w, stream);
   return DLGO_ERR_DTYPE;
-}
-
-// 1 if a kernel of this library gave up a bounded wait since the last call (clears the flag).
-DLGO_EXPORT int dlgo_gemm_simt_error() {
-  int v = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&v, dlgo::g_gemm_split_error, sizeof(int)) != cudaSuccess) return -1;
-  if (v) cudaMemcpyToSymbol(dlgo::g_gemm_split_error, &zero, sizeof(int));
-  return v;
 }

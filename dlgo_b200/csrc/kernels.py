@@ -1398,8 +1398,7 @@ EPI_STORE, EPI_STORE_F32, EPI_ADD_F32 = 0, 1, 2
 
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_STORE,
               out: Optional[torch.Tensor] = None, static_weight: bool = False) -> torch.Tensor:
-    """x[M, K] . w[N, K]^T on the fp32 pipes, or, for more than 16 rows of fp32, by pieces on the tensor cores
-    (csrc/gemm_split.cuh); epilogue stores (x's type or fp32) or adds into fp32 ``out``.
+    """x[M, K] . w[N, K]^T on the fp32 pipes; epilogue stores (x's type or fp32) or adds into fp32 ``out``.
     ``static_weight``: no kernel launched before writes ``w``, so that it may be fetched ahead of their end."""
     _need(w, x.dtype, "w")
     if x.dim() != 2 or x.stride(1) != 1:
@@ -1417,16 +1416,9 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_STORE,
     want = x.dtype if epilogue == EPI_STORE else torch.float32
     if out.dtype != want:
         raise KernelError(f"gemm: out must be {want}")
-    lib = _lib("gemm_simt")
-    scratch = None
-    if M > 16 and x.dtype == torch.float32:
-        lib.dlgo_gemm_simt_scratch.restype = ctypes.c_longlong
-        need = lib.dlgo_gemm_simt_scratch(_ptr(w), _i(dtype_code(x.dtype)), _i(M), _i(N), _i(K), _i(w.stride(0)))
-        if need > 0:
-            scratch = torch.empty((need,), dtype=torch.uint8, device=x.device)
-    st = lib.dlgo_gemm_simt(_ptr(x), _ptr(w), _ptr(out), _i(dtype_code(x.dtype)), _i(M), _i(N), _i(K),
-                            _i(x.stride(0)), _i(w.stride(0)), _i(out.stride(0)), _i(epilogue),
-                            _i(1 if static_weight else 0), _ptr(scratch), _stream())
+    st = _lib("gemm_simt").dlgo_gemm_simt(_ptr(x), _ptr(w), _ptr(out), _i(dtype_code(x.dtype)), _i(M), _i(N), _i(K),
+                                          _i(x.stride(0)), _i(w.stride(0)), _i(out.stride(0)), _i(epilogue),
+                                          _i(1 if static_weight else 0), _stream())
     _check(st, "gemm_simt")
     return out
 
@@ -2115,7 +2107,7 @@ def gemm_tc_rope(x: torch.Tensor, w: torch.Tensor, qkv: torch.Tensor, pair_tile:
 
 def check_device_errors() -> None:
     """Raise if a kernel gave up a bounded wait on the device since the last check (synchronises)."""
-    for lib, fn in (("gemm_tc", "dlgo_gemm_tc_error"), ("gemm_simt", "dlgo_gemm_simt_error"), ("attention_prefill_tc", "dlgo_attention_tc_error"),
+    for lib, fn in (("gemm_tc", "dlgo_gemm_tc_error"), ("attention_prefill_tc", "dlgo_attention_tc_error"),
                     ("moe_tc", "dlgo_moe_tc_error"), ("rglru_tc", "dlgo_rglru_gates_tc_error")):
         if lib in build._loaded:
             v = getattr(build._loaded[lib], fn)()

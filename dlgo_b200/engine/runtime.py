@@ -26,8 +26,7 @@ class Runtime:
 
     ``dtype`` is the type of weights, activations between kernels and the cache:
     ``torch.bfloat16`` (tensor-core contractions, fp32 accumulation) or
-    ``torch.float32`` (everything in true 32-bit: the fp32 pipes, and for
-    prompts' contractions sums of exact products of pieces).  The
+    ``torch.float32`` (everything in true 32-bit on the fp32 pipes).  The
     residual stream, norm statistics, softmax, rotations and logits are fp32 in
     both.
     """

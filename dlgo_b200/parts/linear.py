@@ -2,8 +2,7 @@
 
 The reference keeps matrices row-major ``[out x in]`` and computes one dot
 product per output row (models/llm/model.go:64-80, blas/blas.go:152-196).  In
-float32 the contraction runs on the fp32 pipes (prompts: by exact products of
-pieces on the tensor cores); in bfloat16 on the tensor cores
+float32 the contraction runs on the fp32 pipes; in bfloat16 on the tensor cores
 where the kernel takes the sizes, on the fp32 pipes (bfloat16 operands, fp32
 sums) where it does not.
 """

@@ -117,6 +117,31 @@ def test_gemm_simt_rows_of_both_kernels_are_the_same_sums(M, K_):
         assert torch.equal(k.gemm_simt(x[at:at + n].contiguous(), w, k.EPI_STORE_F32), got[at:at + n])
 
 
+@pytest.mark.parametrize("N,K_", [(1024, 1024), (530, 2052), (300, 4096)])
+def test_gemm_simt_rows_of_large_weights_do_not_depend_on_the_batch(N, K_):
+    """Weights of 2^20 values and more: every row has the bits that it has alone, however many rows come with it."""
+    k = K()
+    x, w = torch.randn(260, K_, device=DEV), torch.randn(N, K_, device=DEV)
+    alone = torch.cat([k.gemm_simt(x[at:at + 1], w, k.EPI_STORE_F32) for at in range(260)])
+    for M in (2, 16, 17, 64, 65, 128, 129, 260):
+        assert torch.equal(k.gemm_simt(x[:M], w, k.EPI_STORE_F32), alone[:M]), M
+
+
+@pytest.mark.parametrize("M", [1, 17, 40, 200])
+def test_gemm_simt_keeps_the_whole_range_of_32_bits(M):
+    """Values next to the smallest normal number, and one product next to the largest.  Each of a running sum's K / 32 = 64
+    additions rounds by 2^-24 / sqrt(3) of what is there (rms), which grows with the square root: 3.3 x 2^-24 of the result,
+    with the sixteen spans' sum 3.7 x 2^-24."""
+    k = K()
+    x, w = torch.randn(M, 2048, device=DEV) * 1e-37, torch.randn(1024, 2048, device=DEV) * 1e20
+    ref = x.double() @ w.double().t()
+    err = k.gemm_simt(x, w, k.EPI_STORE_F32).double() - ref
+    assert err.norm() <= 4 * 2.0 ** -24 * ref.norm()
+    x, w = torch.zeros(M, 2048, device=DEV), torch.zeros(1024, 2048, device=DEV)
+    x[:, 77], w[:, 77] = 3.3893e38, 1.00391
+    assert torch.equal(k.gemm_simt(x, w, k.EPI_STORE_F32), (x[:, 77, None].double() * w[:, 77].double()).float())
+
+
 # --------------------------------------------------------------- rope + append
 def _paged(n_pages, hkv, hd, dtype, fill=float("nan")):
     return (torch.full((n_pages, hkv, 64, hd), fill, device=DEV, dtype=DT[dtype]),
