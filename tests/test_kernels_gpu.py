@@ -1230,11 +1230,12 @@ def test_a_live_position_without_a_page_is_not_written_and_not_read_in_front_of_
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("N", [128, 512])
 @pytest.mark.parametrize("M,K_", [(1, 2048), (9, 2048), (40, 2048), (3, 514), (40, 514)])
-def test_gemm_simt_takes_a_weight_that_the_launch_before_makes(dtype, M, K_):
+def test_gemm_simt_takes_a_weight_that_the_launch_before_makes(dtype, N, M, K_):
     """The launch before says at its start that its successor may begin, and is long: its output is another one each time."""
     k = K()
-    N, dt = 128, DT[dtype]
+    dt = DT[dtype]
     made = torch.zeros(N, K_, device=DEV, dtype=dt)
     wide = torch.randn(K_, 2048, device=DEV).to(dt)
     x = torch.randn(M, K_, device=DEV).to(dt)
