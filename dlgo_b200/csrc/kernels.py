@@ -2359,17 +2359,30 @@ def filter_draw(logits: torch.Tensor, temperature: float, top_k: int, top_p: flo
 _pack_rows = None
 
 
+def _load_pack_rows():
+    """The native reader of lists, or False where it can be neither built nor loaded: Python reads them as well."""
+    try:
+        with build._lock:
+            path = build.ensure_built(["packrows"])["packrows"]
+        # (the interpreter's lock stays held: the numbers are read out of Python objects)
+        fn = ctypes.PyDLL(path).dlgo_pack_rows
+    except (build.KernelBuildError, OSError) as e:
+        build._log(f"note: lists of tokens are read in Python: {e}")
+        return False
+    fn.argtypes = [ctypes.py_object, ctypes.py_object, _i, _p, _ll]
+    fn.restype = _i
+    return fn
+
+
 def pack_rows(parts: list, rows: list, width: int) -> Optional[torch.Tensor]:
     """A list of lists of whole numbers one after another, then the last ``width`` numbers of each of ``rows`` (-1 behind
-    a shorter one), as one int32 tensor on the host; ``None`` where that is not what they are (csrc/packrows.cu).
-    Measured for 64 rows of 64 numbers: 29 us; flattened in Python and packed by ``struct`` 72."""
+    a shorter one), as one int32 tensor on the host; ``None`` where that is not what they are, or the native reader cannot
+    be had (csrc/packrows.cu).  Measured for 64 rows of 64 numbers: 29 us; flattened in Python and packed by ``struct`` 72."""
     global _pack_rows
     if _pack_rows is None:
-        # (the interpreter's lock stays held: the numbers are read out of Python objects)
-        fn = ctypes.PyDLL(build.ensure_built(["packrows"])["packrows"]).dlgo_pack_rows
-        fn.argtypes = [ctypes.py_object, ctypes.py_object, _i, _p, _ll]
-        fn.restype = _i
-        _pack_rows = fn
+        _pack_rows = _load_pack_rows()
+    if not _pack_rows:
+        return None
     room = sum(map(len, parts)) + width * len(rows)
     out = torch.empty((room,), dtype=torch.int32)
     return out if _pack_rows(parts, rows, width, out.data_ptr(), room) == 1 else None

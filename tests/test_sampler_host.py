@@ -60,3 +60,22 @@ def test_numbers_that_are_read_natively():
         assert K.pack_rows(odd, [], 3) is None and K.pack_rows([[1]], odd, 3) is None
     row = iter([1, 2])
     assert K.pack_rows([[1]], [row], 3) is None and list(row) == [1, 2]
+
+
+@pytest.mark.parametrize("error", ["build", "load"])
+def test_lists_are_flattened_where_the_native_reader_cannot_be_had(monkeypatch, tmp_path, error):
+    from dlgo_b200.csrc import build, kernels as K
+    calls = []
+
+    def ensure_built(names, verbose=True):
+        calls.append(names)
+        if error == "build":
+            raise build.KernelBuildError("no compiler")
+        return {n: str(tmp_path / n) for n in names}
+
+    monkeypatch.setattr(K, "_pack_rows", None)
+    monkeypatch.setattr(build, "ensure_built", ensure_built)
+    for _ in range(2):
+        got = _int32_rows(([5, 6], [7, 8]), [[1, 2], [3, 4, 5, 6]], 3, torch.device("cpu"))
+        assert got.tolist() == [5, 6, 7, 8, 1, 2, -1, 4, 5, 6]
+    assert len(calls) == 1          # (asked for once, not for every draw)
