@@ -15,6 +15,9 @@ PyObject* PyList_GetItem(PyObject*, intptr_t);    // borrowed
 long PyLong_AsLong(PyObject*);
 PyObject* PyErr_Occurred(void);
 void PyErr_Clear(void);
+PyObject* PyObject_Type(PyObject*);               // owned
+void Py_DecRef(PyObject*);
+extern struct _typeobject PyList_Type;
 }
 
 namespace {
@@ -32,8 +35,11 @@ bool numbers(PyObject* list, intptr_t from, intptr_t n, int32_t* out) {
   }
   return true;
 }
+// -1 where it is no list, or one of a class of its own, which may give other numbers when it is iterated
 intptr_t size_of(PyObject* o) {
-  const intptr_t n = PyList_Size(o);
+  PyObject* type = PyObject_Type(o);
+  if (type != nullptr) Py_DecRef(type);
+  const intptr_t n = type == (PyObject*)&PyList_Type ? PyList_Size(o) : -1;
   if (n < 0) PyErr_Clear();
   return n;
 }

@@ -79,3 +79,12 @@ def test_lists_are_flattened_where_the_native_reader_cannot_be_had(monkeypatch, 
         got = _int32_rows(([5, 6], [7, 8]), [[1, 2], [3, 4, 5, 6]], 3, torch.device("cpu"))
         assert got.tolist() == [5, 6, 7, 8, 1, 2, -1, 4, 5, 6]
     assert len(calls) == 1          # (asked for once, not for every draw)
+
+
+def test_a_list_of_another_class_is_read_as_it_iterates():
+    class Newest(list):
+        def __iter__(self):
+            return reversed(self)
+
+    got = _int32_rows(([1], [2]), [[3, 4], Newest([5, 6])], 3, torch.device("cpu"))
+    assert got.tolist() == [1, 2, 3, 4, -1, 6, 5, -1]
