@@ -218,14 +218,15 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(AttnParams p) {
 }
 
 // ------------------------------------------------------------------ prompt tiles
-// The same sums for tiles of up to 32 rows (token, query head) of heads of 16 to 128 and pages of 64 keys in one slice, in
-// registers: a thread takes rows 16 apart and, of the scores, 4 keys 16 apart, then the same rows x HD / 16 outputs; the
+// The same sums for tiles of up to 32 rows (token, query head) of heads of 16, 32, 64 or 128 and pages of 64 keys in one slice,
+// in registers: a thread takes rows 16 apart and, of the scores, 4 keys 16 apart, then the same rows x HD / 16 outputs; the
 // sixteen lanes that share a row hold its maximum and its sum.  Keys come 16 bytes at a time from shared memory, for
 // 16 TR multiply-adds per 4 + TR loads; the kernel above loads two words for each multiply-add.  Scores and outputs are
-// summed in the same order as there.
-// Bound by the fp32 pipes where tiles fill the SMs, by the longest tile's chain of pages where they do not (so the tiles
-// that lie late in their sequences begin first).  Measured on a B200, fp32, 32 heads of 64 on 8, two prompts of 366 tokens
-// together: 227 us by the kernel above, 57 here; heads of 16 and prompts of up to 32 tokens 21 and 3.5.
+// summed in the same order as there, a row's weights in another (four of a thread, then sixteen lanes).
+// Bound by the fp32 pipes where tiles fill the SMs, by the longest tile's chain of pages where they do not, so the table's
+// last tiles begin first: a prompt's longest.  (Of several prompts the last one's; two of 65 and 301 tokens take the same time
+// in either order.)  Measured on a B200, fp32, us by the kernel above / here: 32 heads of 64 on 8, prompts of 65 and 301 tokens
+// 214 / 47, one of 1,500 1,883 / 478; 24 heads of 128 on 8 284 / 72 and 3,380 / 851; 4 heads of 16 on 2 55 / 11 and 273 / 77.
 template <int HD, int TR> struct RowsShape {
   static constexpr int ROWS = 16 * TR, KROW = HD + 4, PROW = 80;      // floats from one key / one row's weights to the next
   static constexpr int SMEM = (ROWS * HD + 64 * KROW + 64 * HD + ROWS * PROW) * 4;
